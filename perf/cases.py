@@ -1,0 +1,396 @@
+"""Performance cases: the work a user of this package has it do, each as one
+call sequence through the public entry points.
+
+kind       one pass
+rays       closest hits of a frame's camera rays (pathtracer.trace_rays)
+rebuild    a tree built on the GPU from device triangles, then the frame's
+           camera rays against it (tfgTinyBVHConstruirGPU, trace_rays)
+reference  the drop-in render call with the reference's settings, 1 spp
+           (pathtracer.render_reference_call)
+image      path tracing of `spp` samples into an accumulation buffer
+           (pathtracer.render_pass)
+frame      a frame answered by the radiance cache (nrc.NrcRenderer.frame)
+queries    cache inference (nrc.ColorMLP.inference)
+train      cache training steps, the updated weights read back and a block of
+           queries answered with them (train_step, get_params, inference)
+
+Scenes come from tfg_b200.scenes; a seed changes their proportions, lights,
+camera and frame numbers.  Cache inputs are drawn over the scene bounds with
+the ranges that path tracing produces.
+"""
+import ctypes
+import functools
+import math
+
+import numpy as np
+import torch
+
+from tfg_b200 import _lib, nrc, scenes
+from tfg_b200 import pathtracer as pt
+
+DEV = "cuda"
+LO, HI = (-10.0, -3.0, -18.0), (10.0, 3.0, 2.0)   # cache bounds of the query and training cases
+
+
+def listed():
+    return [
+        # the smallest interactive render: the reference's hand-built room (planes, glass and metal spheres, a small
+        # mesh) through the drop-in call; launches and tails of twenty bounces are all there is
+        dict(name="reference_128", kind="reference", scene="room", size=2, w=128, h=128),
+        # the CPU-sized configuration: displaced icosphere (81,920 triangles) in a box, progressive rendering
+        dict(name="image_512", kind="image", scene="box", size=6, w=512, h=512, spp=4, depth=5),
+        # the headline workload's frame: spheres on terrain (1,000,480 triangles), 1080p, depth 8, a few samples a call
+        dict(name="image_1080p", kind="image", scene="terrain", size=580, w=1920, h=1080, spp=4, depth=8),
+        # primary visibility of that frame as a ray batch
+        dict(name="rays_1080p", kind="rays", scene="terrain", size=580, w=1920, h=1080, tris="watertight"),
+        # geometry that changes: rebuild 81,920 triangles and trace the frame's camera rays
+        dict(name="rebuild_82k", kind="rebuild", scene="box", size=6, w=512, h=512),
+        # one real-time frame with a trained cache, 720p, frame graph on
+        dict(name="frame_720p", kind="frame", scene="terrain", size=290, w=1280, h=720, depth=8, encoding="frequency",
+             width=64, layers=5, precision="fp16"),
+        # a handful of cache queries (tail queries of a small image), a ragged count
+        dict(name="queries_1k", kind="queries", n=1000, encoding="frequency", width=64, layers=5, precision="fp16"),
+        # one query for every pixel of a 1080p frame, the default network
+        dict(name="queries_2m", kind="queries", n=2073600, encoding="frequency", width=64, layers=5, precision="fp16"),
+        # the wide network in BF16, an odd count
+        dict(name="queries_wide", kind="queries", n=230401, encoding="frequency", width=128, layers=5,
+             precision="bf16"),
+        # the reference's own input encoding (hash grid, one-blob, identity) over a 720p frame
+        dict(name="queries_hash", kind="queries", n=921600, encoding="hashgrid", width=64, layers=5,
+             precision="fp16"),
+        # the four training steps of a frame at the default batch
+        dict(name="train_freq", kind="train", n=65536, batch=16384, steps=4, encoding="frequency", width=64, layers=5),
+        # the same with the reference's input encoding
+        dict(name="train_hash", kind="train", n=65536, batch=16384, steps=4, encoding="hashgrid", width=64, layers=5),
+    ]
+
+
+def _log(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def _draw_scene(rng):
+    kind = rng.choice(["box", "terrain"])
+    w = _log(rng, 64, 1920)
+    return dict(scene=kind, size=rng.randint(3, 6) if kind == "box" else 2 * _log(rng, 12, 200), w=w,
+                h=max(36, int(w * rng.uniform(0.5, 0.65))))
+
+
+def _draw_model(rng):
+    return dict(encoding=rng.choice(["frequency", "frequency", "hashgrid"]), width=rng.choice([64, 64, 128]),
+                layers=rng.choice([3, 5, 5, 7]))
+
+
+def draw(rng):
+    kind = rng.choice(["rays", "rebuild", "reference", "image", "image", "frame", "queries", "queries", "train"])
+    if kind == "queries":
+        return dict(kind=kind, n=_log(rng, 200, 2000000), precision=rng.choice(["fp16", "fp16", "bf16", "fp8"]),
+                    **_draw_model(rng))
+    if kind == "train":
+        return dict(kind=kind, n=_log(rng, 2000, 70000), batch=128 * rng.randint(16, 160), steps=rng.randint(1, 4),
+                    **_draw_model(rng))
+    s = _draw_scene(rng)
+    if kind == "rays":
+        return dict(kind=kind, tris=rng.choice(["watertight", "reference"]), **s)
+    if kind == "image":
+        return dict(kind=kind, spp=rng.randint(1, 4), depth=rng.randint(3, 10), **s)
+    if kind == "frame":
+        return dict(kind=kind, depth=rng.randint(4, 8), precision=rng.choice(["fp16", "fp16", "bf16"]),
+                    **_draw_model(rng), **s)
+    if kind == "reference" and rng.random() < 0.5:
+        s.update(scene="room", size=rng.randint(2, 4))
+    return dict(kind=kind, **s)
+
+
+# ---------------------------------------------------------------- inputs
+@functools.lru_cache(maxsize=4)
+def _base(kind, size):
+    """Geometry of one layout and size; the image size and the seed's changes are applied to a copy."""
+    if kind == "room":
+        return scenes.reference_room(64, 64, size)
+    if kind == "box":
+        return scenes.box_icosphere(64, 64, size)
+    return scenes.spheres_terrain(64, 64, subdiv=5 if size > 400 else 4 if size > 150 else 3 if size > 60 else 2,
+                                  terrain_n=size)
+
+
+def _scene(case, seed):
+    base = _base(case["scene"], case["size"])
+    rng = np.random.default_rng([seed, case["w"], case["h"]])
+    mesh = base.mesh.copy()
+    if len(mesh):   # other proportions: every vertex scaled per axis (normals stay close to unit length)
+        mesh["u"][:, :9] *= np.tile(rng.uniform(0.93, 1.07, 3), 3)
+    lights = base.lights.copy()
+    for axis in "xyz":
+        lights["posicion"][axis] += rng.uniform(-0.15, 0.15, len(lights))
+    if case["scene"] == "terrain":
+        cam = scenes.orbit_camera((0.0, -1.0, -7.0), 13.0, 2.8, float(rng.uniform(-20.0, 20.0)), case["w"], case["h"])
+    else:
+        eye = (float(rng.uniform(-0.3, 0.3)), -0.75 + float(rng.uniform(-0.2, 0.2)), 4.25)
+        cam = scenes.make_camera(eye, (0.0, -0.75, 0.0), width=case["w"], height=case["h"])
+    return scenes.Scene(base.prims, mesh, lights, cam, case["w"], case["h"], bounds=base.bounds, name=base.name)
+
+
+def _rows(n, seed):
+    """n cache rows (112 B): positions over the bounds, directions and normals mapped to [0, 1], albedos, targets."""
+    g = torch.Generator(DEV).manual_seed(seed)
+    rows = torch.zeros((n, 14), dtype=torch.float64, device=DEV)
+    lo = torch.tensor(LO, dtype=torch.float64, device=DEV)
+    hi = torch.tensor(HI, dtype=torch.float64, device=DEV)
+    pos = torch.rand((n, 3), generator=g, device=DEV, dtype=torch.float64)
+    rows[:, 0:3] = (lo + (hi - lo) * pos).float()
+    for k in (3, 6):
+        d = torch.randn((n, 3), generator=g, device=DEV)
+        rows[:, k:k + 3] = d / d.norm(dim=1, keepdim=True) * 0.5 + 0.5
+    f = rows.view(torch.float32)   # float columns 18..26: diffuse, specular, target colour
+    f[:, 18:24] = torch.rand((n, 6), generator=g, device=DEV) * 0.8 + 0.1
+    shade = 0.5 + 0.5 * torch.sin(3.0 * pos.sum(1, keepdim=True)).float()
+    f[:, 24:27] = shade * f[:, 18:21] * (0.5 + torch.rand((n, 3), generator=g, device=DEV))
+    return rows
+
+
+def _weights(case, seed):
+    """Layer weights, flat and padded as the model keeps them, and the hash-grid tables (or None)."""
+    rng = np.random.default_rng([seed, 77])
+    live = 63 if case["encoding"] == "hashgrid" else 85
+    shapes = nrc.layer_shapes(case["layers"], case["width"])
+    out = []
+    for k, (r, c) in enumerate(shapes):
+        w = np.zeros((r, c), np.float32)
+        nr, nc = 3 if k == len(shapes) - 1 else r, live if k == 0 else c
+        w[:nr, :nc] = rng.uniform(-1.0, 1.0, (nr, nc)) * math.sqrt(6.0 / (nr + nc))
+        out.append(w.reshape(-1))
+    table = None
+    if case["encoding"] == "hashgrid":
+        table = rng.random(16 * 2 ** 19 * 2, dtype=np.float32) - np.float32(0.5)
+    return np.concatenate(out), table
+
+
+def _model(case, seed, bounds=(LO, HI)):
+    mlp = nrc.ColorMLP(batch=case.get("batch", 16384), hidden_layers=case["layers"], width=case["width"],
+                       encoding=nrc.HASHGRID if case["encoding"] == "hashgrid" else nrc.FREQUENCY)
+    w, table = _weights(case, seed)
+    mlp.set_params(w)
+    if table is not None:
+        mlp.set_table(table)
+    mlp.set_bounds(*bounds)
+    return mlp
+
+
+def _precision(mlp, case, rows, n):
+    p = case.get("precision", "fp16")
+    if p == "fp8":
+        mlp.calibrate(rows, min(n, 16384))
+    mlp.set_precision({"fp16": nrc.FP16, "bf16": nrc.BF16, "fp8": nrc.FP8}[p])
+
+
+def prepare(case, seed):
+    kind, st = case["kind"], {"kind": case["kind"]}
+    if kind == "queries":
+        st["n"], st["rows"] = case["n"], _rows(case["n"], seed)
+        st["mlp"] = _model(case, seed)
+        st["out"] = torch.zeros((case["n"], 3), dtype=torch.float32, device=DEV)
+        _precision(st["mlp"], case, st["rows"], case["n"])
+        return st
+    if kind == "train":
+        st["n"], st["steps"], st["rows"] = case["n"], case["steps"], _rows(case["n"], seed)
+        st["mlp"] = _model(case, seed)
+        st["probe"] = _rows(4096, seed + 1000003)
+        st["out"] = torch.zeros((4096, 3), dtype=torch.float32, device=DEV)
+        return st
+    W, H = case["w"], case["h"]
+    scene = _scene(case, seed)
+    st["frame"] = seed % 1000
+    if kind == "rebuild":
+        st["mesh"] = torch.from_numpy(scene.mesh.view(np.uint8)).to(DEV)
+        st["n"] = len(scene.mesh)
+        scene = scenes.Scene(scene.prims, scene.mesh[:0], scene.lights, scene.camera, W, H, bounds=scene.bounds)
+    ds = st["ds"] = pt.DeviceScene(scene, DEV)
+    if kind in ("rays", "rebuild"):
+        st["rays"] = torch.empty(W * H * 8, dtype=torch.float32, device=DEV)
+        pt.camera_rays_ex(ds, st["frame"], 1, pt.RAYS_TILES, st["rays"])
+        st["hits"] = torch.zeros((W * H, 4), dtype=torch.float32, device=DEV)
+        st["tris"] = pt.TRIS_REF if case.get("tris") == "reference" else pt.TRIS_WATERTIGHT
+    elif kind == "frame":
+        prm = pt.RenderParams(max_depth=case["depth"], rr_min_depth=3, shadow_mesh=1, tri_format=pt.TRIS_WATERTIGHT)
+        st["mlp"] = _model(case, seed, scene.bounds)
+        _precision(st["mlp"], case, None, 0)
+        st["renderer"] = nrc.NrcRenderer(ds, st["mlp"], prm, train_steps=0)
+    else:
+        st["img"] = torch.zeros((H, W, 3), dtype=torch.float32, device=DEV)
+        if kind == "image":
+            st["accum"] = torch.zeros((H, W, 3), dtype=torch.float32, device=DEV)
+            st["params"] = pt.RenderParams(max_depth=case["depth"], rr_min_depth=3, shadow_mesh=1,
+                                           tri_format=pt.TRIS_WATERTIGHT, spp=case["spp"], accumulate=1)
+        else:
+            st["nrc"] = pt.NrcBuffers(W * H, DEV)
+    return st
+
+
+# ---------------------------------------------------------------- one pass
+def run(st):
+    kind = st["kind"]
+    if kind == "queries":
+        st["mlp"].inference(st["rows"], st["out"], st["n"])
+        return st["out"]
+    if kind == "train":
+        for _ in range(st["steps"]):
+            st["mlp"].train_step(st["rows"], st["n"], read_loss=False)
+        st["mlp"].inference(st["probe"], st["out"], 4096)
+        return {"weights": st["mlp"].get_params(nrc.WEIGHTS), "answers": st["out"]}
+    ds, frame = st["ds"], st["frame"]
+    if kind in ("rays", "rebuild"):
+        if kind == "rebuild":
+            _lib.lib.tfgTinyBVHLiberar(ctypes.byref(ds.bvh))
+            _lib.call("tfgTinyBVHConstruirGPU", st["mesh"].data_ptr(), st["n"], ctypes.byref(ds.bvh),
+                      torch.cuda.current_stream().cuda_stream)
+        pt.trace_rays(ds, st["rays"], st["hits"], st["tris"])
+        return {"tuv": st["hits"][:, :3], "id": st["hits"].view(torch.int32)[:, 3]}
+    if kind == "frame":
+        r = st["renderer"]
+        r.frame(frame, accumulate=True)
+        st["frame"] += 1
+        return {"img": r.img, "accum": r.accum}
+    if kind == "image":
+        pt.render_pass(ds, st["params"], frame, st["img"], st["accum"])
+        st["frame"] += st["params"].spp
+        return {"img": st["img"], "accum": st["accum"]}
+    pt.render_reference_call(ds, frame, st["img"], st["nrc"])
+    st["frame"] += 1
+    return st["img"]
+
+
+# ---------------------------------------------------------------- what a pass cannot do without
+def _layer_macs(case):
+    return sum(r * c for r, c in nrc.layer_shapes(case["layers"], case["width"]))
+
+
+def _triangles(case):
+    if case["scene"] == "terrain":
+        s = case["size"]
+        return 2 * s * s + 16 * 20 * 4 ** (5 if s > 400 else 4 if s > 150 else 3 if s > 60 else 2)
+    return 20 * 4 ** case["size"]
+
+
+def work(case):
+    kind = case["kind"]
+    if kind in ("queries", "train"):
+        macs = _layer_macs(case)
+        levels = 16 * 8 * 4 * 2.0 if case["encoding"] == "hashgrid" else 0.0   # corner blends of two features
+        if kind == "queries":
+            return {"bytes": case["n"] * 124.0 + 2.0 * macs, "flops": case["n"] * (2.0 * macs + levels)}
+        samples = float(case["batch"] * case["steps"])
+        state = macs + (16 * 2 ** 19 * 2 if case["encoding"] == "hashgrid" else 0)
+        # weights, moments and average read and written by every step; rows read once per sample
+        return {"bytes": samples * 112.0 + case["steps"] * state * 32.0 + 4096 * 124.0,
+                "flops": samples * (6.0 * macs + 3.0 * levels) + 4096 * (2.0 * macs + levels)}
+    px, tris = float(case["w"] * case["h"]), float(_triangles(case))
+    tree = tris * (48.0 + 8.0)                      # watertight triangles and nodes, each read once
+    ray = 10 * 8 * 12.0 + 4 * 40.0                  # ten nodes of eight boxes and four triangles
+    if kind == "rays":
+        return {"bytes": px * 48.0 + tree, "flops": px * ray}
+    if kind == "rebuild":
+        return {"bytes": tris * (200.0 + 200.0 + 64.0 + 48.0 + 8.0) + px * 48.0 + tree,
+                "flops": px * ray + tris * 500.0}
+    spp = case.get("spp", 1)
+    out = px * (12.0 if kind == "reference" else 36.0)
+    nrc_flops = px * 2.0 * _layer_macs(case) if kind == "frame" else 0.0
+    return {"bytes": out + tree + min(tris, px * spp) * 200.0, "flops": px * spp * 4.0 * ray + nrc_flops}
+
+
+# ---------------------------------------------------------------- 64-bit values
+def _features(case, rows, table):
+    """Layer-0 inputs in 64 bits (96 columns)."""
+    f = rows.view(torch.float32).double()
+    lo = torch.tensor(LO, dtype=torch.float64, device=DEV)
+    hi = torch.tensor(HI, dtype=torch.float64, device=DEV)
+    p = ((rows[:, 0:3] - lo) / (hi - lo)).clamp(0.0, 1.0)
+    n = len(rows)
+    one = torch.ones((n, 1), dtype=torch.float64, device=DEV)
+    if case["encoding"] != "hashgrid":
+        ang = p[:, :, None] * (math.pi * 2.0 ** torch.arange(12, dtype=torch.float64, device=DEV))
+        bands = torch.stack([ang.sin(), ang.cos()], dim=3).reshape(n, 72)
+        x = torch.cat([bands, rows[:, 3:9], f[:, 18:24], one], 1)
+    else:
+        feats = []
+        for level in range(16):
+            cells = math.floor(16.0 * 1.5 ** level)
+            s = p * cells
+            c = torch.minimum(s.floor(), torch.full_like(s, cells - 1.0))
+            w, c = s - c, c.long()
+            acc = 0.0
+            for k in range(8):
+                q = [c[:, a] + ((k >> a) & 1) for a in range(3)]
+                if (cells + 1) ** 3 <= 2 ** 19:
+                    idx = q[0] + (cells + 1) * (q[1] + (cells + 1) * q[2])
+                else:
+                    idx = (q[0] ^ (q[1] * 2654435761) ^ (q[2] * 805459861)) & (2 ** 19 - 1)
+                wk = 1.0
+                for a in range(3):
+                    wk = wk * (w[:, a] if (k >> a) & 1 else 1.0 - w[:, a])
+                acc = acc + wk[:, None] * table[level * 2 ** 19 + idx]
+            feats.append(acc)
+        edge = (torch.arange(5, dtype=torch.float64, device=DEV) / 4.0 - rows[:, 3:9, None]) * 4.0
+        cdf = 0.5 * (1.0 + torch.erf(edge / math.sqrt(2.0)))
+        x = torch.cat(feats + [(cdf[:, :, 1:] - cdf[:, :, :-1]).reshape(n, 24), f[:, 18:24], one], 1)
+    return torch.nn.functional.pad(x, (0, 96 - x.shape[1]))
+
+
+def _forward(case, ws, rows, table):
+    x = _features(case, rows, table)
+    for w in ws[:-1]:
+        x = torch.relu(x @ w.T)
+    return (x @ ws[-1].T)[:, :3]
+
+
+def _layers64(case, flat):
+    out, o = [], 0
+    for r, c in nrc.layer_shapes(case["layers"], case["width"]):
+        out.append(torch.from_numpy(flat[o:o + r * c]).to(DEV).double().view(r, c))
+        o += r * c
+    return out
+
+
+def _answers(case, ws, rows, table):
+    with torch.no_grad():
+        return torch.cat([_forward(case, ws, r, table).clamp(0.0, 1e5) for r in rows.split(1 << 17)])
+
+
+def _picked(step, batch, n):
+    """Rows a training step draws: a PCG output of (step ^ sample), modulo the record count."""
+    m = 0xFFFFFFFF
+    s = (np.arange(batch, dtype=np.uint64) ^ np.uint64(step)) * np.uint64(747796405) + np.uint64(2891336453) & np.uint64(m)
+    w = ((s >> ((s >> np.uint64(28)) + np.uint64(4))) ^ s) * np.uint64(277803737) & np.uint64(m)
+    return torch.from_numpy((((w >> np.uint64(22)) ^ w) % np.uint64(n)).astype(np.int64)).to(DEV)
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind not in ("queries", "train"):
+        return None   # path tracing: a branch taken the other way in 64 bits gives another path
+    flat, table = _weights(case, seed)
+    if table is not None:
+        table = torch.from_numpy(table).to(DEV).double().view(-1, 2)
+    ws = _layers64(case, flat)
+    if kind == "queries":
+        return _answers(case, ws, _rows(case["n"], seed), table)
+    rows = _rows(case["n"], seed)
+    par = ws + ([table] if table is not None else [])
+    m, v, ema = ([torch.zeros_like(p) for p in par] for _ in range(3))
+    for step in range(case["steps"]):
+        sel = rows[_picked(step, case["batch"], case["n"])]
+        y = sel.view(torch.float32)[:, 24:27].double()
+        leaves = [p.clone().requires_grad_(True) for p in par]
+        out = _forward(case, leaves[:len(ws)], sel, leaves[-1] if table is not None else None)
+        lum = out.detach() @ torch.tensor([0.299, 0.587, 0.114], dtype=torch.float64, device=DEV)
+        loss = ((out - y) ** 2 / (lum[:, None] ** 2 + 0.01)).mean()
+        for k, g in enumerate(torch.autograd.grad(loss, leaves)):
+            m[k] = 0.9 * m[k] + 0.1 * g
+            v[k] = 0.99 * v[k] + 0.01 * g * g
+            t = step + 1
+            par[k] = par[k] - 1e-2 * (m[k] / (1.0 - 0.9 ** t)) / ((v[k] / (1.0 - 0.99 ** t)).sqrt() + 1e-15)
+            ema[k] = 0.99 * ema[k] + 0.01 * par[k]
+    avg = [e / (1.0 - 0.99 ** case["steps"]) for e in ema]
+    probe = _rows(4096, seed + 1000003)
+    answers = _answers(case, avg[:len(ws)], probe, avg[-1] if table is not None else None)
+    return {"weights": torch.cat([p.reshape(-1) for p in par[:len(ws)]]), "answers": answers}
