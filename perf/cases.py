@@ -177,6 +177,12 @@ def _model(case, seed, bounds=(LO, HI)):
     return mlp
 
 
+@functools.lru_cache(maxsize=1)
+def _frame_stream():
+    """The one stream on which a program runs its cache frames, whichever renderer they belong to."""
+    return torch.cuda.Stream(DEV)
+
+
 def _precision(mlp, case, rows, n):
     p = case.get("precision", "fp16")
     if p == "fp8":
@@ -215,7 +221,7 @@ def prepare(case, seed):
         prm = pt.RenderParams(max_depth=case["depth"], rr_min_depth=3, shadow_mesh=1, tri_format=pt.TRIS_WATERTIGHT)
         st["mlp"] = _model(case, seed, scene.bounds)
         _precision(st["mlp"], case, None, 0)
-        st["renderer"] = nrc.NrcRenderer(ds, st["mlp"], prm, train_steps=0)
+        st["renderer"] = nrc.NrcRenderer(ds, st["mlp"], prm, train_steps=0, stream=_frame_stream())
     else:
         st["img"] = torch.zeros((H, W, 3), dtype=torch.float32, device=DEV)
         if kind == "image":
@@ -368,6 +374,8 @@ def exact(case, seed):
     kind = case["kind"]
     if kind not in ("queries", "train"):
         return None   # path tracing: a branch taken the other way in 64 bits gives another path
+    if case.get("precision") == "fp8":
+        return None   # E4M3 operands: the answers are a tenth or so away from the 64-bit network's
     flat, table = _weights(case, seed)
     if table is not None:
         table = torch.from_numpy(table).to(DEV).double().view(-1, 2)
