@@ -328,10 +328,13 @@ int tfgGenerateCameraRays(const TfgCamara* camara, int32_t ancho_img, int32_t al
  * Every setting computes the same image from the same inputs (bit for bit);
  * only speed and memory change. */
 typedef struct TfgRenderTuning {
-    int32_t wavefront_paths;    /* queue capacity: paths per wavefront, 0 (default) = one sample of every
-                                   pixel (W*H).  More runs several samples of the call per launch, less
-                                   splits a sample into chunks; passes that query or train the cache
-                                   stop at W*H.  0 or 1024 .. 2^26 (224 B of device memory per path) */
+    int32_t wavefront_paths;    /* queue capacity: paths per wavefront.  0 (default) = the call's samples
+                                   spread evenly over wavefronts of at most 2^24 paths and an eighth of
+                                   the free device memory, at least one sample of every pixel (W*H) --
+                                   exactly one under stream capture.  More runs several samples of the
+                                   call per launch, less splits a sample into chunks; passes that query
+                                   or train the cache stop at W*H.  0 or 1024 .. 2^26 (224 B of device
+                                   memory per path) */
     int32_t trace_threads;      /* threads per traversal and shadow-ray CTA: 64, 128 (default) or 256 */
     int32_t trace_warps_per_sm; /* resident traversal warps per SM; 0 (default) = as many as fit */
     int32_t refill_min;         /* idle lanes that make a traversal warp fetch new rays, 1..32 (default 8) */

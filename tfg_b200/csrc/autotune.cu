@@ -61,9 +61,9 @@ int time_tuning(int dev, const TuneScene& sc, const TfgRenderTuning& t, int repe
 std::vector<int32_t> candidates(int k, uint32_t npix, uint64_t paths) {
     std::vector<int32_t> v;
     switch (k) {
-        case 0: {   // wavefront: 1/8 .. 16 samples of the image, 0 = exactly one
+        case 0: {   // wavefront: 1/8 .. 16 samples of the image, 0 = the library's choice
             v.push_back(0);
-            const uint64_t sizes[] = {npix / 8u, npix / 4u, npix / 2u, 2ull * npix, 4ull * npix, 8ull * npix,
+            const uint64_t sizes[] = {npix / 8u, npix / 4u, npix / 2u, npix, 2ull * npix, 4ull * npix, 8ull * npix,
                                       16ull * npix};
             for (uint64_t w : sizes)
                 if (w >= 1024 && w <= (1u << 26) && w <= paths) v.push_back((int32_t)w);

@@ -255,7 +255,7 @@ def profile_get() -> dict:
 class RenderTuning:
     """TfgRenderTuning: how the wavefront stages are sized and launched on the
     current device.  Every setting renders the same image."""
-    wavefront_paths: int = 0      # queue capacity in paths; 0 = one sample of the image (W*H)
+    wavefront_paths: int = 0      # queue capacity in paths; 0 = whole samples of the image, up to 2^24 paths
     trace_threads: int = 128      # threads per traversal / shadow CTA: 64, 128, 256
     trace_warps_per_sm: int = 0   # resident traversal warps per SM; 0 = as many as fit
     refill_min: int = 8           # idle lanes that make a traversal warp fetch new rays
