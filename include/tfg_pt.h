@@ -167,7 +167,8 @@ int  tfgTinyBVHConstruir(const TfgPrimitiva* primitivas_host, int32_t n, TfgTiny
  * Morton-ordered binary tree (Karras 2012), collapsed to 8-wide nodes and
  * quantised on the device; same node / triangle layouts as
  * tfgTinyBVHConstruir, a lower-quality (LBVH) tree that builds in
- * milliseconds.  Synchronises `stream`; free with tfgTinyBVHLiberar. */
+ * milliseconds.  Synchronises `stream`; free with tfgTinyBVHLiberar (the
+ * arrays share an allocation). */
 int  tfgTinyBVHConstruirGPU(const TfgPrimitiva* primitivas_device, int32_t n, TfgTinyBVH* out, void* stream);
 /* Frees what tfgTinyBVHConstruir / tfgTinyBVHConstruirGPU allocated (TinyBVH::~TinyBVH). */
 void tfgTinyBVHLiberar(TfgTinyBVH* bvh);

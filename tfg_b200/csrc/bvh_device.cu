@@ -5,11 +5,44 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/tfg_pt.h"
 #include "tfg_errors.h"
+#include "tfg_runtime.h"
+
+namespace tfg {
+namespace {
+
+// Live results that are one allocation starting at the primitives, made by
+// tfgTinyBVHConstruirGPU.
+std::mutex g_blocks_mutex;
+std::vector<const void*> g_blocks;
+
+// Takes a result that starts at `prims` off the list; false when its arrays
+// are allocations of their own.
+bool take_block(const void* prims) {
+    if (!prims) return false;
+    std::lock_guard<std::mutex> lk(g_blocks_mutex);
+    for (size_t i = 0; i < g_blocks.size(); ++i)
+        if (g_blocks[i] == prims) {
+            g_blocks[i] = g_blocks.back();
+            g_blocks.pop_back();
+            return true;
+        }
+    return false;
+}
+
+}  // namespace
+
+void bvh_register_block(const void* prims) {
+    std::lock_guard<std::mutex> lk(g_blocks_mutex);
+    g_blocks.push_back(prims);
+}
+
+}  // namespace tfg
 
 extern "C" int tfgTinyBVHConstruir(const TfgPrimitiva* prims, int32_t n, TfgTinyBVH* out) {
     if (!out) return tfg::fail(TFG_E_INVALID, "tfgTinyBVHConstruir: out is null");
@@ -56,9 +89,17 @@ extern "C" int tfgTinyBVHConstruir(const TfgPrimitiva* prims, int32_t n, TfgTiny
 
 extern "C" void tfgTinyBVHLiberar(TfgTinyBVH* b) {
     if (!b) return;
-    if (b->ref.d_nodos) cudaFree(b->ref.d_nodos);
-    if (b->ref.d_tris) cudaFree(b->ref.d_tris);
-    if (b->d_tris_wt) cudaFree(b->d_tris_wt);
-    if (b->d_primitivas) cudaFree(b->d_primitivas);
+    if (tfg::take_block(b->d_primitivas)) {
+        // nodes that did not fit the block are an allocation of their own
+        const char* block = reinterpret_cast<const char*>(b->d_primitivas);
+        const char* wt_end = reinterpret_cast<const char*>(b->d_tris_wt) + ((size_t)b->num_primitivas * 48 + 255) / 256 * 256;
+        if (b->ref.d_nodos && reinterpret_cast<const char*>(b->ref.d_nodos) != wt_end) cudaFree(b->ref.d_nodos);
+        cudaFree(const_cast<char*>(block));
+    } else {
+        if (b->ref.d_nodos) cudaFree(b->ref.d_nodos);
+        if (b->ref.d_tris) cudaFree(b->ref.d_tris);
+        if (b->d_tris_wt) cudaFree(b->d_tris_wt);
+        if (b->d_primitivas) cudaFree(b->d_primitivas);
+    }
     std::memset(b, 0, sizeof(*b));
 }

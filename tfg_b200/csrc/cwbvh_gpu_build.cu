@@ -9,25 +9,36 @@
 //   3. binary radix tree over the sorted codes (Karras 2012, "Maximizing
 //      Parallelism in the Construction of BVHs, Octrees, and k-d Trees"),
 //      duplicate codes ordered by index;
-//   4. boxes and triangle counts bottom-up, one thread per leaf climbing
-//      while it is the second child to finish;
-//   5. one kernel per wide level: every wide node gathers up to 8 children
-//      by opening the largest-area interior child (a subtree of <= 3
-//      triangles becomes a leaf slot), assigns octant slots greedily,
-//      quantises the child boxes to 8 bits and reserves contiguous blocks
-//      for its inner children and leaf triangles with atomics;
+//   4. boxes, triangle counts and collapse plans bottom-up, one thread per
+//      leaf climbing while it is the second child to finish;
+//   5. one kernel per wide level, eight lanes per wide node: the lanes expand
+//      the node's collapse plan into its up to 8 children (a subtree of <= 3
+//      triangles becomes a leaf slot), assign octant slots greedily, quantise
+//      the child boxes to 8 bits and reserve contiguous blocks for the inner
+//      children and leaf triangles with atomics;
 //   6. the reference transform triangles and the watertight triangles in
 //      leaf order.
-// The tree is a Morton-order (LBVH) tree: it builds in milliseconds, and
-// traverses slower than the host builder's binned-SAH tree.
+// The tree is a Morton-order (LBVH) tree: it builds in under a millisecond
+// for 10^5 triangles, and traverses slower than the host builder's binned-SAH
+// tree.
+//
+// A build is a chain of short dependent kernels, so what counts is the host
+// work around them and each kernel's latency: all scratch is one block of a
+// bounded stream-ordered pool (cudaMalloc and cudaFree take ~0.3 ms each here:
+// the former 25 pairs took most of the 5.8 ms of an 81,920-triangle build),
+// the result is one allocation made while the GPU works, the initial values
+// come from a kernel, and the levels run in batches whose sizes stay on the
+// device (one host read per eight levels instead of one per level).
 #include <cuda_runtime.h>
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 
 #include "../../include/tfg_pt.h"
@@ -39,24 +50,32 @@ namespace {
 
 constexpr int kMaxLeaf = 3;   // the 3-bit unary meta count limits a leaf to 3 triangles
 
-struct Box6 {
-    float lo[3], hi[3];
+// Box and triangle count of a binary node (or of a triangle), read and
+// written as two 16-byte halves.
+struct __align__(16) BNode {
+    float lo[3];
+    int count;
+    float hi[3];
+    float pad;
 };
 
-// Collapse plan of a binary node, as in the host builder (cwbvh_build.cpp):
-// for a budget of i = 1..8 slots of the wide parent, the least SAH cost of
-// the node's subtree and how it is reached (leaf of <= 3 triangles, a wide
-// node of its own, as with one slot less, or split with k slots to the left).
-struct Plan2 {
+// Collapse plan of an interior binary node, as in the host builder
+// (cwbvh_build.cpp): for a budget of i = 1..8 slots of the wide parent, the
+// least SAH cost of the node's subtree and how it is reached (leaf of <= 3
+// triangles, a wide node of its own, as with one slot less, or split with k
+// slots to the left).  A single triangle has no stored plan: every budget
+// costs its leaf.
+struct __align__(16) Plan2 {
     float cost[8];
     uint8_t how[8];
     uint8_t split8;       // as a wide node: slots given to the left child
     uint8_t pad[7];
 };
+static_assert(sizeof(BNode) == 32 && sizeof(Plan2) == 48, "vector loads");
 constexpr uint8_t kLeaf = 0, kInternal = 1, kSame = 2, kSplit = 16;
 constexpr float kCostWideNode = 1.0f, kCostWideTri = 0.3f;
 
-__device__ __forceinline__ float box_area(const Box6& b) {
+__device__ __forceinline__ float box_area(const BNode& b) {
     const float dx = fmaxf(b.hi[0] - b.lo[0], 0.0f), dy = fmaxf(b.hi[1] - b.lo[1], 0.0f),
                 dz = fmaxf(b.hi[2] - b.lo[2], 0.0f);
     return 2.0f * (dx * dy + dx * dz + dy * dz);
@@ -70,34 +89,9 @@ __device__ __forceinline__ uint32_t expand_bits(uint32_t v) {   // 10 bits -> ev
     return v;
 }
 
-__global__ void k_flag_triangles(const TfgPrimitiva* __restrict__ p, int n, uint32_t* __restrict__ flag) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        flag[i] = p[i].tipo == TFG_TRIANGULO ? 1u : 0u;
-}
-
-// Compacted triangles: primitive copy, FP32 vertices, box.
-__global__ void k_compact(const TfgPrimitiva* __restrict__ p, int n, const uint32_t* __restrict__ flag,
-                          const uint32_t* __restrict__ pos, TfgPrimitiva* __restrict__ tris, float* __restrict__ verts,
-                          Box6* __restrict__ box) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (!flag[i]) continue;
-        const uint32_t k = pos[i];
-        tris[k] = p[i];
-        const auto& t = p[i].u.triangulo;
-        const TfgVec3d* v[3] = {&t.v0, &t.v1, &t.v2};
-        Box6 b;
-        for (int a = 0; a < 3; ++a) { b.lo[a] = INFINITY; b.hi[a] = -INFINITY; }
-        for (int c = 0; c < 3; ++c) {
-            const float x[3] = {(float)v[c]->x, (float)v[c]->y, (float)v[c]->z};
-            for (int a = 0; a < 3; ++a) {
-                verts[9 * (size_t)k + 3 * c + a] = x[a];
-                b.lo[a] = fminf(b.lo[a], x[a]);
-                b.hi[a] = fmaxf(b.hi[a], x[a]);
-            }
-        }
-        box[k] = b;
-    }
-}
+struct IsTriangle {
+    __host__ __device__ uint32_t operator()(const TfgPrimitiva& p) const { return p.tipo == TFG_TRIANGULO ? 1u : 0u; }
+};
 
 // Order-preserving float <-> uint mapping for atomic min / max.
 __device__ __forceinline__ uint32_t fkey(float f) {
@@ -108,32 +102,102 @@ __device__ __forceinline__ float funkey(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
 
-__global__ void k_centroid_bounds(const Box6* __restrict__ box, uint32_t n, uint32_t* __restrict__ cb) {
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+// Device words of one build.
+struct BuildWords {
+    uint32_t cb[6];             // centroid bounds as ordered keys: lo.xyz, hi.xyz
+    uint32_t next_node, next_tri;
+    uint32_t level[66];         // wide nodes of each level
+};
+
+// Initial values: empty centroid bounds, the root as the only node of level
+// 0 (binary node 0; with one triangle, its leaf), nothing arrived.
+__global__ void k_build_init(BuildWords* w, int2* q0, uint32_t* arrivals, uint32_t nt) {
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t i = i0; i < nt; i += gridDim.x * blockDim.x) arrivals[i] = 0u;
+    if (i0 < 6) w->cb[i0] = i0 < 3 ? 0xFFFFFFFFu : 0u;
+    if (i0 == 6) w->next_node = 1u;
+    if (i0 == 7) w->next_tri = 0u;
+    if (i0 >= 8 && i0 < 8 + 66) w->level[i0 - 8] = i0 == 8 ? 1u : 0u;
+    if (i0 == 74) *q0 = make_int2(0, 0);
+}
+
+// Compacted triangles' FP32 vertices and boxes, and the centroid bounds.
+// `pos` counts the triangles up to and including each primitive.
+__global__ void __launch_bounds__(256) k_compact(const TfgPrimitiva* __restrict__ p, int n,
+                                                 const uint32_t* __restrict__ pos, float* __restrict__ verts,
+                                                 BNode* __restrict__ box, BuildWords* words) {
+    float clo[3] = {INFINITY, INFINITY, INFINITY}, chi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (p[i].tipo != TFG_TRIANGULO) continue;
+        const uint32_t k = pos[i] - 1u;
+        const auto& t = p[i].u.triangulo;
+        const TfgVec3d* v[3] = {&t.v0, &t.v1, &t.v2};
+        BNode b;
+        for (int a = 0; a < 3; ++a) { b.lo[a] = INFINITY; b.hi[a] = -INFINITY; }
+        for (int c = 0; c < 3; ++c) {
+            const float x[3] = {(float)v[c]->x, (float)v[c]->y, (float)v[c]->z};
+            for (int a = 0; a < 3; ++a) {
+                verts[9 * (size_t)k + 3 * c + a] = x[a];
+                b.lo[a] = fminf(b.lo[a], x[a]);
+                b.hi[a] = fmaxf(b.hi[a], x[a]);
+            }
+        }
+        b.count = 1;
+        b.pad = 0.0f;
+        box[k] = b;
         for (int a = 0; a < 3; ++a) {
-            const float c = 0.5f * (box[i].lo[a] + box[i].hi[a]);
-            lo[a] = fminf(lo[a], c);
-            hi[a] = fmaxf(hi[a], c);
+            const float c = 0.5f * (b.lo[a] + b.hi[a]);
+            clo[a] = fminf(clo[a], c);
+            chi[a] = fmaxf(chi[a], c);
         }
+    }
+    __shared__ uint32_t s_cb[6];
+    if (threadIdx.x < 6) s_cb[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+    __syncthreads();
     for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xFFFFFFFFu, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xFFFFFFFFu, hi[a], o));
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&cb[a], fkey(lo[a]));
-            atomicMax(&cb[3 + a], fkey(hi[a]));
+        const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, fkey(clo[a])), hi = __reduce_max_sync(0xFFFFFFFFu, fkey(chi[a]));
+        if ((threadIdx.x & 31) == 0) { atomicMin(&s_cb[a], lo); atomicMax(&s_cb[3 + a], hi); }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(&words->cb[threadIdx.x], s_cb[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(&words->cb[threadIdx.x], s_cb[threadIdx.x]);
+}
+
+// The TRIANGULO primitives, compacted.  A warp copies the 200-byte structs of
+// its 32 primitives together, 8 bytes per lane and step (a struct per lane
+// moves them at a 200-byte stride).
+__global__ void __launch_bounds__(256) k_copy_prims(const TfgPrimitiva* __restrict__ p, int n,
+                                                    const uint32_t* __restrict__ pos, TfgPrimitiva* __restrict__ tris) {
+    constexpr int kWords = (int)(sizeof(TfgPrimitiva) / 8);
+    const int lane = threadIdx.x & 31;
+    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base < n; base += gridDim.x * blockDim.x) {
+        const int i = base + lane;
+        const bool tri = i < n && p[i].tipo == TFG_TRIANGULO;
+        const uint32_t k = tri ? pos[i] - 1u : 0u;
+        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, tri);
+        const unsigned long long* src = reinterpret_cast<const unsigned long long*>(p + base);
+        if (mask == 0xFFFFFFFFu) {
+            unsigned long long* dst =
+                reinterpret_cast<unsigned long long*>(tris + __shfl_sync(0xFFFFFFFFu, k, 0));
+#pragma unroll
+            for (int w = 0; w < kWords; ++w) dst[32 * w + lane] = __ldg(&src[32 * w + lane]);
+        } else {
+            for (uint32_t m = mask; m; m &= m - 1u) {
+                const int j = __ffs(m) - 1;
+                unsigned long long* dst =
+                    reinterpret_cast<unsigned long long*>(tris + __shfl_sync(0xFFFFFFFFu, k, j));
+                if (lane < kWords) dst[lane] = __ldg(&src[kWords * j + lane]);
+            }
         }
     }
 }
 
-__global__ void k_morton(const Box6* __restrict__ box, uint32_t n, const uint32_t* __restrict__ cb,
+__global__ void k_morton(const BNode* __restrict__ box, uint32_t n, const BuildWords* __restrict__ words,
                          uint32_t* __restrict__ code, uint32_t* __restrict__ idx) {
     float lo[3], inv[3];
     for (int a = 0; a < 3; ++a) {
-        lo[a] = funkey(cb[a]);
-        const float ext = funkey(cb[3 + a]) - lo[a];
+        lo[a] = funkey(words->cb[a]);
+        const float ext = funkey(words->cb[3 + a]) - lo[a];
         inv[a] = ext > 0.0f ? 1.0f / ext : 0.0f;
     }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -148,14 +212,14 @@ __global__ void k_morton(const Box6* __restrict__ box, uint32_t n, const uint32_
 }
 
 // Binary radix tree: internal nodes 0..n-2, leaf i (sorted position) is node
-// n - 1 + i.  child[2i], child[2i+1]; parent of every node.
+// n - 1 + i.  child[i] = (left, right); parent of every node.
 __device__ __forceinline__ int delta_of(const uint32_t* code, int n, int i, int j) {
     if (j < 0 || j >= n) return -1;
     const uint32_t a = code[i], b = code[j];
     return a == b ? 32 + __clz((uint32_t)(i ^ j)) : __clz(a ^ b);
 }
 
-__global__ void k_radix_tree(const uint32_t* __restrict__ code, int n, int* __restrict__ child,
+__global__ void k_radix_tree(const uint32_t* __restrict__ code, int n, int2* __restrict__ child,
                              int* __restrict__ parent) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
         const int d = (delta_of(code, n, i, i + 1) - delta_of(code, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -175,93 +239,126 @@ __global__ void k_radix_tree(const uint32_t* __restrict__ code, int n, int* __re
         const int gamma = i + s * d + min(d, 0);
         const int left = min(i, j) == gamma ? (n - 1 + gamma) : gamma;
         const int right = max(i, j) == gamma + 1 ? (n - 1 + gamma + 1) : gamma + 1;
-        child[2 * i] = left;
-        child[2 * i + 1] = right;
+        child[i] = make_int2(left, right);
         parent[left] = i;
         parent[right] = i;
     }
 }
 
-// Boxes and triangle counts bottom-up.  A thread stops at the first node whose
-// other child is not finished yet; the second thread to arrive continues.
-// The plan of binary node p from its area, triangle count and its children's
-// plans (C(n, 1) = min(leaf, wide node); C(n, i) = min(C(n, i - 1), D(n, i));
+// The plan of a binary node from its area, triangle count and its children's
+// costs (C(n, 1) = min(leaf, wide node); C(n, i) = min(C(n, i - 1), D(n, i));
 // D(n, j) = min over k of C(left, k) + C(right, j - k)).
-__device__ void plan_node(Plan2& P, float area, int count, const Plan2* L, const Plan2* R) {
+__device__ __forceinline__ void plan_node(Plan2& P, float area, int count, const float (&lc)[8], const float (&rc)[8]) {
     float dist[9];
     uint8_t split[9];
-    for (int j = 0; j <= 8; ++j) { dist[j] = INFINITY; split[j] = 0; }
-    if (L && R) {
-        float lc[8], rc[8];
-        for (int k = 0; k < 8; ++k) { lc[k] = __ldcg(&L->cost[k]); rc[k] = __ldcg(&R->cost[k]); }
-        for (int j = 2; j <= 8; ++j)
-            for (int k = 1; k < j; ++k) {
-                const float c = lc[k - 1] + rc[j - k - 1];
-                if (c < dist[j]) { dist[j] = c; split[j] = (uint8_t)k; }
-            }
+#pragma unroll
+    for (int j = 2; j <= 8; ++j) {
+        dist[j] = INFINITY;
+        split[j] = 0;
+#pragma unroll
+        for (int k = 1; k < j; ++k) {
+            const float c = lc[k - 1] + rc[j - k - 1];
+            if (c < dist[j]) { dist[j] = c; split[j] = (uint8_t)k; }
+        }
     }
     const float leaf = count <= kMaxLeaf ? area * (float)count * kCostWideTri : INFINITY;
     const float internal = dist[8] + area * kCostWideNode;
     P.split8 = split[8];
     if (leaf <= internal) { P.cost[0] = leaf; P.how[0] = kLeaf; }
     else { P.cost[0] = internal; P.how[0] = kInternal; }
+#pragma unroll
     for (int i = 2; i <= 8; ++i) {
         if (dist[i] < P.cost[i - 2]) { P.cost[i - 1] = dist[i]; P.how[i - 1] = (uint8_t)(kSplit + split[i]); }
         else { P.cost[i - 1] = P.cost[i - 2]; P.how[i - 1] = kSame; }
     }
 }
 
-__global__ void k_refit(const Box6* __restrict__ tbox, const uint32_t* __restrict__ sorted, int n,
-                        const int* __restrict__ child, const int* __restrict__ parent, Box6* box, int* count,
-                        Plan2* plan, uint32_t* arrivals) {
+__device__ __forceinline__ bool is_leaf2(int node, int n) { return node >= n - 1; }
+
+__device__ __forceinline__ BNode load_node(const BNode* b) {   // written by another thread of this kernel
+    const float4* q = reinterpret_cast<const float4*>(b);
+    const float4 x = __ldcg(q), y = __ldcg(q + 1);
+    BNode r;
+    r.lo[0] = x.x; r.lo[1] = x.y; r.lo[2] = x.z; r.count = __float_as_int(x.w);
+    r.hi[0] = y.x; r.hi[1] = y.y; r.hi[2] = y.z; r.pad = 0.0f;
+    return r;
+}
+
+// Boxes, counts and plans bottom-up.  A thread stops at the first node whose
+// other child is not finished yet; the second thread to arrive continues, its
+// own child's box and costs in registers, and reads only the sibling's.  The
+// chain of ~20 such steps is latency (atomic, fence, sibling): 16-byte loads
+// issued together and no plans stored for single triangles.
+__global__ void __launch_bounds__(256) k_refit(const BNode* __restrict__ tbox, const uint32_t* __restrict__ sorted,
+                                               int n, const int2* __restrict__ child, const int* __restrict__ parent,
+                                               BNode* box, Plan2* plan, uint32_t* arrivals) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int node = n - 1 + i;
-        box[node] = tbox[sorted[i]];
-        count[node] = 1;
-        plan_node(plan[node], box_area(tbox[sorted[i]]), 1, nullptr, nullptr);
-        __threadfence();
+        BNode own = tbox[sorted[i]];
+        box[node] = own;
+        float cost[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) cost[k] = box_area(own) * 1.0f * kCostWideTri;
         while (node != 0) {
             const int p = parent[node];
+            const int2 c = child[p];
+            __threadfence();
             if (atomicAdd(&arrivals[p], 1u) == 0u) break;
             __threadfence();
-            const int a = child[2 * p], b = child[2 * p + 1];
-            Box6 ba, bb, r;
-            for (int k = 0; k < 3; ++k) {
-                ba.lo[k] = __ldcg(&box[a].lo[k]); ba.hi[k] = __ldcg(&box[a].hi[k]);
-                bb.lo[k] = __ldcg(&box[b].lo[k]); bb.hi[k] = __ldcg(&box[b].hi[k]);
-                r.lo[k] = fminf(ba.lo[k], bb.lo[k]);
-                r.hi[k] = fmaxf(ba.hi[k], bb.hi[k]);
+            const bool left = c.x == node;
+            const int sib = left ? c.y : c.x;
+            const BNode o = load_node(&box[sib]);
+            float oc[8];
+            if (is_leaf2(sib, n)) {
+                const float l = box_area(o) * 1.0f * kCostWideTri;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) oc[k] = l;
+            } else {
+                const float4* q = reinterpret_cast<const float4*>(plan[sib].cost);
+                const float4 x = __ldcg(q), y = __ldcg(q + 1);
+                oc[0] = x.x; oc[1] = x.y; oc[2] = x.z; oc[3] = x.w;
+                oc[4] = y.x; oc[5] = y.y; oc[6] = y.z; oc[7] = y.w;
             }
+            BNode r;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                r.lo[k] = fminf(own.lo[k], o.lo[k]);
+                r.hi[k] = fmaxf(own.hi[k], o.hi[k]);
+            }
+            r.count = own.count + o.count;
+            r.pad = 0.0f;
             box[p] = r;
-            const int cnt = __ldcg(&count[a]) + __ldcg(&count[b]);
-            count[p] = cnt;
-            plan_node(plan[p], box_area(r), cnt, &plan[a], &plan[b]);
-            __threadfence();
+            float lc[8], rc[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) { lc[k] = left ? cost[k] : oc[k]; rc[k] = left ? oc[k] : cost[k]; }
+            Plan2 P;
+            plan_node(P, box_area(r), r.count, lc, rc);
+#pragma unroll
+            for (int k = 0; k < 7; ++k) P.pad[k] = 0;
+            plan[p] = P;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) cost[k] = P.cost[k];
+            own = r;
             node = p;
         }
     }
 }
 
 struct WideArgs {
-    const int* child;
-    const Box6* box;
-    const int* count;
+    const int2* child;
+    const BNode* box;
     const Plan2* plan;
     const uint32_t* sorted;   // sorted position -> compacted triangle index
     int n;                    // triangles
+    int level;
     const int2* q_in;         // (binary node, wide index)
-    uint32_t q_n;
     int2* q_out;
-    uint32_t* q_out_n;
-    uint32_t* next_node;
-    uint32_t* next_tri;
+    BuildWords* words;
     uint32_t* nodes;          // 20 words per wide node
     uint32_t* tri_order;      // leaf order -> compacted triangle index
 };
 
-__device__ __forceinline__ bool is_leaf2(int node, int n) { return node >= n - 1; }
-
-__device__ int gather_leaf_tris(const WideArgs& a, int node, uint32_t* out) {
+__device__ int gather_leaf_tris(const WideArgs& a, int node, uint32_t (&out)[kMaxLeaf]) {
     int stack[8], sp = 0, cnt = 0;
     stack[sp++] = node;
     while (sp > 0 && cnt < kMaxLeaf) {
@@ -269,140 +366,210 @@ __device__ int gather_leaf_tris(const WideArgs& a, int node, uint32_t* out) {
         if (is_leaf2(m, a.n)) {
             out[cnt++] = a.sorted[m - (a.n - 1)];
         } else {
-            stack[sp++] = a.child[2 * m + 1];
-            stack[sp++] = a.child[2 * m];
+            const int2 c = a.child[m];
+            stack[sp++] = c.y;
+            stack[sp++] = c.x;
         }
     }
     return cnt;
 }
 
-// One wide node per thread: the host builder's cost-optimal collapse (read
-// from the plans), slot assignment and quantisation (cwbvh_build.cpp) on this
-// level's queue.
-__global__ void k_wide_level(WideArgs a) {
-    const uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (qi >= a.q_n) return;
-    const int node2 = a.q_in[qi].x;
-    const uint32_t widx = (uint32_t)a.q_in[qi].y;
-    int kid[8];
-    bool leaf[8];
-    int nk = 0;
-    if (is_leaf2(node2, a.n)) {
-        kid[0] = node2; leaf[0] = true; nk = 1;
-    } else {
-        // (binary node, slot budget) pairs, the left child on top; a split
-        // pushes two entries and pops one, and the budgets sum to 8, so the
-        // stack never holds more than 8
-        int sn[8], sb[8], sp = 0;
-        const int k8 = a.plan[node2].split8;
-        sn[sp] = a.child[2 * node2 + 1]; sb[sp++] = 8 - k8;
-        sn[sp] = a.child[2 * node2]; sb[sp++] = k8;
-        while (sp > 0 && nk < 8) {
-            const int m = sn[--sp];
-            int b = sb[sp];
-            const Plan2& P = a.plan[m];
-            while (b > 1 && P.how[b - 1] == kSame) --b;
-            const uint8_t h = P.how[b - 1];
-            if (h == kLeaf || h == kInternal) {
-                kid[nk] = m; leaf[nk] = h == kLeaf; ++nk;
-            } else if (sp + 2 <= 8) {
-                const int k = h - kSplit;
-                sn[sp] = a.child[2 * m + 1]; sb[sp++] = b - k;
-                sn[sp] = a.child[2 * m]; sb[sp++] = k;
+// 2^e as a double, e in [-1022, 1023].
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
+// Exponent of the quantisation step along one axis: the smallest e >= -126
+// with 255 * 2^e >= ext (0 extent: -126), at most 127.
+__device__ __forceinline__ int grid_exponent(double ext) {
+    int ex = -126;
+    if (ext > 0.0) {
+        ex = (int)ceil(log2(ext / 255.0));
+        while (ldexp(255.0, ex) < ext) ++ex;
+        ex = max(ex, -126);
+    }
+    return min(ex, 127);
+}
+
+// One wide node per eight lanes: the host builder's cost-optimal collapse
+// (read from the plans), slot assignment and quantisation (cwbvh_build.cpp)
+// on this level's queue.  A level's time is one node's latency while the
+// levels are small, so a node's work is spread over its lanes: they hold its
+// children left to right and open all open ones in each round (a thread per
+// node walked the plan child by child, kept 64 double costs in local memory
+// and took 51 us per level of an 81,920-triangle build).
+constexpr int kWideThreads = 128;
+
+__global__ void __launch_bounds__(kWideThreads) k_wide_level(WideArgs a) {
+    __shared__ int4 s_item[kWideThreads / 8][8];       // (binary node, budget or lane, state, -)
+    __shared__ __align__(16) uint32_t s_node[kWideThreads / 8][20];
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    const uint32_t qn = a.words->level[a.level];
+    const uint32_t lane = threadIdx.x & 31u, j = threadIdx.x & 7u, g = threadIdx.x >> 3, g0 = lane & 24u;
+    const uint32_t stride = gridDim.x * (kWideThreads / 8);
+    for (uint32_t base = blockIdx.x * (kWideThreads / 8) + (threadIdx.x >> 5) * 4u; base < qn; base += stride) {
+        const bool act = base + (lane >> 3) < qn;
+        int node2 = 0, widx = 0;
+        if (act) { const int2 q = a.q_in[base + (lane >> 3)]; node2 = q.x; widx = q.y; }
+        // ---- children: lane j holds the j-th from the left
+        int item = -1, budget = 0, nk = 0;
+        bool leaf = false, open = false;
+        if (act) {
+            if (is_leaf2(node2, a.n)) {
+                nk = 1;
+                if (j == 0) { item = node2; leaf = true; }
+            } else {
+                // (no split was finite over non-finite boxes: split8 = 0)
+                const int k8 = a.plan[node2].split8 ? a.plan[node2].split8 : 4;
+                const int2 c = a.child[node2];
+                nk = 2;
+                if (j < 2) { item = j == 0 ? c.x : c.y; budget = j == 0 ? k8 : 8 - k8; open = true; }
             }
         }
-    }
-    const Box6 pb = a.box[node2];
-    // Octant slot assignment, greedy on dot(c_child - c_parent, dir_s).
-    double pc[3];
-    for (int k = 0; k < 3; ++k) pc[k] = 0.5 * ((double)pb.lo[k] + (double)pb.hi[k]);
-    double cost[8][8];
-    for (int i = 0; i < nk; ++i) {
-        const Box6 cb = a.box[kid[i]];
+        while (__any_sync(kFull, open)) {
+            bool split = false;
+            int kl = 0;
+            int2 c = make_int2(0, 0);
+            if (open) {
+                if (is_leaf2(item, a.n)) {
+                    leaf = true;
+                    open = false;
+                } else {
+                    const uint2 how = *reinterpret_cast<const uint2*>(a.plan[item].how);
+                    c = a.child[item];
+                    auto at = [&](int b) { return ((b < 4 ? how.x : how.y) >> (8 * (b & 3))) & 0xFFu; };
+                    while (budget > 1 && at(budget - 1) == kSame) --budget;
+                    const uint32_t h = at(budget - 1);
+                    if (h == kLeaf || h == kInternal) {
+                        leaf = h == kLeaf;
+                        open = false;
+                    } else {
+                        split = true;
+                        kl = (int)h - kSplit;
+                    }
+                }
+            }
+            const uint32_t sm = (__ballot_sync(kFull, split) >> g0) & 0xFFu;
+            const int at = (int)j + __popc(sm & ((1u << j) - 1u));
+            if ((int)j < nk) {
+                s_item[g][at] = make_int4(split ? c.x : item, split ? kl : budget, (open ? 1 : 0) | (leaf ? 2 : 0), 0);
+                if (split) s_item[g][at + 1] = make_int4(c.y, budget - kl, 1, 0);
+            }
+            nk += __popc(sm);
+            __syncwarp();
+            if ((int)j < nk) {
+                const int4 v = s_item[g][j];
+                item = v.x; budget = v.y; open = v.z & 1; leaf = (v.z & 2) != 0;
+            }
+            __syncwarp();
+        }
+        // ---- octant slots, greedy on dot(c_child - c_parent, dir_s): the
+        // least cost, then the leftmost child, then the lowest slot
+        const bool kid = act && (int)j < nk;
+        BNode pb{}, cb{};
+        if (act) pb = a.box[node2];
+        if (kid) cb = a.box[item];
         double d[3];
-        for (int k = 0; k < 3; ++k) d[k] = 0.5 * ((double)cb.lo[k] + (double)cb.hi[k]) - pc[k];
-        for (int s = 0; s < 8; ++s)
-            cost[i][s] = d[0] * ((s & 4) ? -1.0 : 1.0) + d[1] * ((s & 2) ? -1.0 : 1.0) + d[2] * ((s & 1) ? -1.0 : 1.0);
-    }
-    int slot_of[8], kid_in_slot[8];
-    for (int s = 0; s < 8; ++s) { kid_in_slot[s] = -1; slot_of[s] = -1; }
-    for (int round = 0; round < nk; ++round) {
-        double best = INFINITY;
-        int bi = -1, bs = -1;
-        for (int i = 0; i < nk; ++i) {
-            if (slot_of[i] >= 0) continue;
-            for (int s = 0; s < 8; ++s) {
-                if (kid_in_slot[s] >= 0) continue;
-                if (cost[i][s] < best || bi < 0) { best = cost[i][s]; bi = i; bs = s; }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            d[k] = 0.5 * ((double)cb.lo[k] + (double)cb.hi[k]) - 0.5 * ((double)pb.lo[k] + (double)pb.hi[k]);
+        uint32_t taken = 0;
+        int slot = -1;
+        while (__any_sync(kFull, kid && slot < 0)) {
+            double best = INFINITY;
+            int bs = -1;
+            if (kid && slot < 0) {
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const double c = d[0] * ((s & 4) ? -1.0 : 1.0) + d[1] * ((s & 2) ? -1.0 : 1.0) +
+                                     d[2] * ((s & 1) ? -1.0 : 1.0);
+                    if (!((taken >> s) & 1u) && (c < best || bs < 0)) { best = c; bs = s; }
+                }
+            }
+            int bj = bs < 0 ? 8 : (int)j;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const double ob = __shfl_xor_sync(kFull, best, o);
+                const int oj = __shfl_xor_sync(kFull, bj, o), os = __shfl_xor_sync(kFull, bs, o);
+                if (oj < 8 && (bj == 8 || ob < best || (ob == best && oj < bj))) { best = ob; bj = oj; bs = os; }
+            }
+            bj = __shfl_sync(kFull, bj, 0, 8);   // one lane's choice for the group, whatever the costs
+            bs = __shfl_sync(kFull, bs, 0, 8);
+            if (bj < 8) {
+                taken |= 1u << bs;
+                if (bj == (int)j) slot = bs;
             }
         }
-        slot_of[bi] = bs;
-        kid_in_slot[bs] = bi;
-    }
-    // Quantisation grid.
-    float p[3];
-    int e[3];
-    for (int k = 0; k < 3; ++k) {
-        p[k] = pb.lo[k];
-        const double ext = (double)pb.hi[k] - (double)pb.lo[k];
-        int ex = -126;
-        if (ext > 0.0) {
-            ex = (int)ceil(log2(ext / 255.0));
-            while (ldexp(255.0, ex) < ext) ++ex;
-            ex = max(ex, -126);
-        }
-        e[k] = min(ex, 127);
-    }
-    // Reserve the inner children's node block and the leaf triangles' block.
-    uint32_t inner = 0, ntri = 0;
-    uint32_t leaf_tris[8][kMaxLeaf];
-    int leaf_cnt[8];
-    for (int i = 0; i < nk; ++i) {
-        leaf_cnt[i] = 0;
-        if (leaf[i]) { leaf_cnt[i] = gather_leaf_tris(a, kid[i], leaf_tris[i]); ntri += (uint32_t)leaf_cnt[i]; }
-        else ++inner;
-    }
-    const uint32_t child_base = inner ? atomicAdd(a.next_node, inner) : 0u;
-    const uint32_t tri_base = ntri ? atomicAdd(a.next_tri, ntri) : 0u;
-    const uint32_t qbase = inner ? atomicAdd(a.q_out_n, inner) : 0u;
-    uint8_t meta[8] = {0}, qlo[3][8] = {{0}}, qhi[3][8] = {{0}};
-    uint32_t imask = 0, rank = 0, toff = 0;
-    for (int s = 0; s < 8; ++s) {
-        const int i = kid_in_slot[s];
-        if (i < 0) continue;
-        const Box6 cb = a.box[kid[i]];
+        // ---- lane j takes the child in slot j
+        s_item[g][j] = make_int4(-1, (int)j, 0, 0);
+        __syncwarp();
+        if (kid) s_item[g][slot] = make_int4(item, (int)j, leaf ? 2 : 0, 0);
+        __syncwarp();
+        const int4 mine = s_item[g][j];
+        const bool has = mine.x >= 0;
+        leaf = has && (mine.z & 2) != 0;
+        const bool inner = has && !leaf;
+        float lo[3], hi[3];
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const double step = ldexp(1.0, e[k]);
-            const double lo = floor(((double)cb.lo[k] - (double)p[k]) / step);
-            const double hi = ceil(((double)cb.hi[k] - (double)p[k]) / step);
-            qlo[k][s] = (uint8_t)fmin(fmax(lo, 0.0), 255.0);
-            qhi[k][s] = (uint8_t)fmin(fmax(hi, 0.0), 255.0);
+            lo[k] = __shfl_sync(kFull, cb.lo[k], mine.y, 8);
+            hi[k] = __shfl_sync(kFull, cb.hi[k], mine.y, 8);
         }
-        if (leaf[i]) {
-            const uint32_t c = (uint32_t)leaf_cnt[i];
-            meta[s] = (uint8_t)((((1u << c) - 1u) << 5) | toff);
-            for (uint32_t k = 0; k < c; ++k) a.tri_order[tri_base + toff + k] = leaf_tris[i][k];
-            toff += c;
-        } else {
-            imask |= 1u << s;
-            meta[s] = (uint8_t)((1u << 5) | (24u + (uint32_t)s));
-            a.q_out[qbase + rank] = make_int2(kid[i], (int)(child_base + rank));
-            ++rank;
+        uint32_t tri[kMaxLeaf];
+        const int cnt = leaf ? gather_leaf_tris(a, mine.x, tri) : 0;
+        // ---- reserve the inner children's node block and the leaf triangles' block
+        const uint32_t im = __ballot_sync(kFull, inner);
+        int tsum = cnt;   // running triangle count over the warp's slots
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, tsum, o);
+            if ((int)lane >= o) tsum += v;
         }
-    }
-    uint32_t* w = a.nodes + 20 * (size_t)widx;
-    w[0] = __float_as_uint(p[0]); w[1] = __float_as_uint(p[1]); w[2] = __float_as_uint(p[2]);
-    w[3] = (uint32_t)(uint8_t)(int8_t)e[0] | ((uint32_t)(uint8_t)(int8_t)e[1] << 8) |
-           ((uint32_t)(uint8_t)(int8_t)e[2] << 16) | (imask << 24);
-    w[4] = inner ? child_base : 0u;
-    w[5] = 4u * tri_base;
-    auto pack4 = [](const uint8_t* b) {
-        return (uint32_t)b[0] | ((uint32_t)b[1] << 8) | ((uint32_t)b[2] << 16) | ((uint32_t)b[3] << 24);
-    };
-    w[6] = pack4(meta); w[7] = pack4(meta + 4);
-    for (int k = 0; k < 3; ++k) {
-        w[8 + 2 * k] = pack4(qlo[k]); w[9 + 2 * k] = pack4(qlo[k] + 4);
-        w[14 + 2 * k] = pack4(qhi[k]); w[15 + 2 * k] = pack4(qhi[k] + 4);
+        const uint32_t ni = (uint32_t)__popc(im), nt = (uint32_t)__shfl_sync(kFull, tsum, 31);
+        uint32_t r0 = 0, r1 = 0, r2 = 0;
+        if (lane == 0) {
+            if (ni) { r0 = atomicAdd(&a.words->next_node, ni); r2 = atomicAdd(&a.words->level[a.level + 1], ni); }
+            if (nt) r1 = atomicAdd(&a.words->next_tri, nt);
+        }
+        r0 = __shfl_sync(kFull, r0, 0);
+        r1 = __shfl_sync(kFull, r1, 0);
+        r2 = __shfl_sync(kFull, r2, 0);
+        const uint32_t gi = (im >> g0) & 0xFFu;                                   // the node's inner slots
+        const uint32_t ibefore = (uint32_t)__popc(im & ((1u << g0) - 1u));        // inner children of earlier nodes
+        const uint32_t rank = (uint32_t)__popc(gi & ((1u << j) - 1u));
+        const uint32_t tfirst = (uint32_t)(__shfl_sync(kFull, tsum, (int)g0) - __shfl_sync(kFull, cnt, (int)g0));
+        const uint32_t gtris = (uint32_t)__shfl_sync(kFull, tsum, (int)g0 + 7) - tfirst;
+        const uint32_t toff = (uint32_t)(tsum - cnt) - tfirst;
+        const uint32_t child_base = gi ? r0 + ibefore : 0u, tri_base = gtris ? r1 + tfirst : 0u;
+        // ---- quantisation and the node's 80 bytes
+        uint8_t* nb = reinterpret_cast<uint8_t*>(s_node[g]);
+        const int axis = j < 2 ? (int)j : 2;
+        const int ej = grid_exponent((double)(axis == 0 ? pb.hi[0] : axis == 1 ? pb.hi[1] : pb.hi[2]) -
+                                     (double)(axis == 0 ? pb.lo[0] : axis == 1 ? pb.lo[1] : pb.lo[2]));
+        int e[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            e[k] = __shfl_sync(kFull, ej, k, 8);
+            const double inv = pow2(-e[k]);
+            const double ql = floor(((double)lo[k] - (double)pb.lo[k]) * inv);
+            const double qh = ceil(((double)hi[k] - (double)pb.lo[k]) * inv);
+            nb[32 + 8 * k + j] = has ? (uint8_t)fmin(fmax(ql, 0.0), 255.0) : (uint8_t)0;
+            nb[56 + 8 * k + j] = has ? (uint8_t)fmin(fmax(qh, 0.0), 255.0) : (uint8_t)0;
+        }
+        nb[24 + j] = leaf ? (uint8_t)((((1u << cnt) - 1u) << 5) | toff) : inner ? (uint8_t)((1u << 5) | (24u + j)) : (uint8_t)0;
+        if (j == 0) {
+            uint32_t* w = s_node[g];
+            w[0] = __float_as_uint(pb.lo[0]); w[1] = __float_as_uint(pb.lo[1]); w[2] = __float_as_uint(pb.lo[2]);
+            w[3] = (uint32_t)(uint8_t)(int8_t)e[0] | ((uint32_t)(uint8_t)(int8_t)e[1] << 8) |
+                   ((uint32_t)(uint8_t)(int8_t)e[2] << 16) | (gi << 24);
+            w[4] = child_base;
+            w[5] = 4u * tri_base;
+        }
+        if (leaf)
+            for (int k = 0; k < cnt; ++k) a.tri_order[tri_base + toff + (uint32_t)k] = tri[k];
+        if (inner) a.q_out[r2 + ibefore + rank] = make_int2(mine.x, (int)(child_base + rank));
+        __syncwarp();
+        if (act && j < 5)
+            reinterpret_cast<uint4*>(a.nodes + 20 * (size_t)widx)[j] = reinterpret_cast<const uint4*>(s_node[g])[j];
+        __syncwarp();
     }
 }
 
@@ -412,10 +579,10 @@ __global__ void k_emit_tris(const float* __restrict__ verts, const uint32_t* __r
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nt; k += gridDim.x * blockDim.x) {
         const uint32_t t = order[k];
         const float* tv = &verts[9 * (size_t)t];
-        float* W = &tris_wt[12 * (size_t)k];
-        W[0] = tv[0]; W[1] = tv[1]; W[2] = tv[2]; W[3] = __uint_as_float(t);
-        W[4] = tv[3]; W[5] = tv[4]; W[6] = tv[5]; W[7] = 0.0f;
-        W[8] = tv[6]; W[9] = tv[7]; W[10] = tv[8]; W[11] = 0.0f;
+        float4* W = reinterpret_cast<float4*>(tris_wt) + 3 * (size_t)k;
+        W[0] = make_float4(tv[0], tv[1], tv[2], __uint_as_float(t));
+        W[1] = make_float4(tv[3], tv[4], tv[5], 0.0f);
+        W[2] = make_float4(tv[6], tv[7], tv[8], 0.0f);
         const double v0[3] = {tv[0], tv[1], tv[2]};
         const double e1[3] = {tv[3] - v0[0], tv[4] - v0[1], tv[5] - v0[2]};
         const double e2[3] = {tv[6] - v0[0], tv[7] - v0[1], tv[8] - v0[2]};
@@ -427,10 +594,10 @@ __global__ void k_emit_tris(const float* __restrict__ verts, const uint32_t* __r
         double nrm[3], r0[3], r1[3];
         cross(e1, e2, nrm);
         const double n2 = nrm[0] * nrm[0] + nrm[1] * nrm[1] + nrm[2] * nrm[2];
-        float* R = &tris_ref[16 * (size_t)k];
+        float4* R = reinterpret_cast<float4*>(tris_ref) + 4 * (size_t)k;
         if (!(n2 > 0.0) || !isfinite(n2)) {
-            for (int j = 0; j < 12; ++j) R[j] = 0.0f;
-            R[11] = 1.0f;
+            R[0] = R[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            R[2] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
         } else {
             cross(e2, nrm, r0);
             cross(nrm, e1, r1);
@@ -439,33 +606,63 @@ __global__ void k_emit_tris(const float* __restrict__ verts, const uint32_t* __r
             for (int c = 0; c < 3; ++c) { rows[0][c] = r0[c] * inv; rows[1][c] = r1[c] * inv; rows[2][c] = nrm[c] * inv; }
             for (int r = 0; r < 3; ++r) {
                 const double wv = -(rows[r][0] * v0[0] + rows[r][1] * v0[1] + rows[r][2] * v0[2]);
-                R[4 * r + 0] = (float)rows[r][0];
-                R[4 * r + 1] = (float)rows[r][1];
-                R[4 * r + 2] = (float)rows[r][2];
-                R[4 * r + 3] = (float)wv;
+                R[r] = make_float4((float)rows[r][0], (float)rows[r][1], (float)rows[r][2], (float)wv);
             }
         }
-        R[12] = 0.0f; R[13] = 0.0f; R[14] = 0.0f; R[15] = __uint_as_float(t);
+        R[3] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(t));
     }
 }
 
-// Scratch of one build, freed on every exit path.
+// Pool of each device that builds' scratch blocks come from: stream-ordered,
+// keeping at most kPoolKeep bytes between builds (more goes back to the
+// device when a build's stream has been synchronised).  One block per build,
+// so builds on several threads or streams never share memory.
+constexpr uint64_t kPoolKeep = 128ull << 20;
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pool[kMaxDevices] = {nullptr};
+
+cudaError_t build_pool(int dev, cudaMemPool_t* out) {
+    std::lock_guard<std::mutex> lk(g_pool_mutex);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        uint64_t keep = kPoolKeep;
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+            if (pool) cudaMemPoolDestroy(pool);
+            return e;
+        }
+        g_pool[dev] = pool;
+    }
+    *out = g_pool[dev];
+    return cudaSuccess;
+}
+
+// One scratch block, carved into 256-byte aligned arrays; freed in stream
+// order on every exit path.
 struct Scratch {
-    static constexpr int kSlots = 32;
-    void* p[kSlots] = {nullptr};
-    int n = 0;
-    cudaError_t err = cudaSuccess;
+    cudaStream_t s;
+    uint8_t* base = nullptr;
+    size_t used = 0;
+    explicit Scratch(cudaStream_t st) : s(st) {}
+    cudaError_t reserve(cudaMemPool_t pool, size_t bytes) {
+        return cudaMallocFromPoolAsync((void**)&base, bytes, pool, s);
+    }
+    static size_t pad(size_t bytes) { return (bytes + 255) & ~size_t(255); }
     template <typename T>
     T* get(size_t count) {
-        if (err != cudaSuccess) return nullptr;
-        if (n == kSlots) { err = cudaErrorMemoryAllocation; return nullptr; }
-        void* q = nullptr;
-        err = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-        if (err == cudaSuccess) p[n++] = q;
-        return static_cast<T*>(q);
+        T* q = reinterpret_cast<T*>(base + used);
+        used += pad(count * sizeof(T));
+        return q;
     }
     ~Scratch() {
-        for (int i = 0; i < n; ++i) cudaFree(p[i]);
+        if (base) cudaFreeAsync(base, s);
     }
 };
 
@@ -483,118 +680,127 @@ extern "C" int tfgTinyBVHConstruirGPU(const TfgPrimitiva* d_prims, int32_t n, Tf
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return fail((int)e, cudaGetErrorString(e));
     if (int rc = require_sm100(dev)) return rc;
-    const uint32_t blocks = std::min<uint32_t>(((uint32_t)n + 255) / 256, 148u * 8u);
-    Scratch sc;
-    uint32_t* flag = sc.get<uint32_t>(n);
-    uint32_t* pos = sc.get<uint32_t>(n);
-    size_t tmp_bytes = 0;
-    if (sc.err == cudaSuccess) sc.err = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, flag, pos, n, s);
-    void* tmp = sc.get<uint8_t>(tmp_bytes);
-    if (sc.err != cudaSuccess) return fail((int)sc.err, std::string("tfgTinyBVHConstruirGPU: ") + cudaGetErrorString(sc.err));
-    k_flag_triangles<<<blocks, 256, 0, s>>>(d_prims, n, flag);
-    if (sc.err == cudaSuccess) sc.err = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flag, pos, n, s);
-    uint32_t nt = 0, last_flag = 0;
-    if (sc.err == cudaSuccess) sc.err = cudaMemcpyAsync(&nt, pos + n - 1, 4, cudaMemcpyDeviceToHost, s);
-    if (sc.err == cudaSuccess) sc.err = cudaMemcpyAsync(&last_flag, flag + n - 1, 4, cudaMemcpyDeviceToHost, s);
-    if (sc.err == cudaSuccess) sc.err = cudaStreamSynchronize(s);
-    if (sc.err != cudaSuccess) return fail((int)sc.err, std::string("tfgTinyBVHConstruirGPU: ") + cudaGetErrorString(sc.err));
-    nt += last_flag;
-    if (nt == 0) return ok();   // no triangles: an empty BVH, as the host path
-    if (nt > (1u << 29)) return fail(TFG_E_INVALID, "tfgTinyBVHConstruirGPU: too many triangles");
-
-    TfgPrimitiva* tris = nullptr;
-    e = cudaMalloc((void**)&tris, (size_t)nt * sizeof(TfgPrimitiva));
-    if (e != cudaSuccess) return fail((int)e, std::string("tfgTinyBVHConstruirGPU: ") + cudaGetErrorString(e));
-    out->d_primitivas = tris;
-    out->num_primitivas = nt;
     auto bail = [&](cudaError_t err) {
         tfgTinyBVHLiberar(out);
         return fail((int)err, std::string("tfgTinyBVHConstruirGPU: ") + cudaGetErrorString(err));
     };
+    cudaMemPool_t pool = nullptr;
+    e = build_pool(dev, &pool);
+    if (e != cudaSuccess) return bail(e);
+    // how many triangles there are: the last value of a running count
+    const auto flags = thrust::make_transform_iterator(d_prims, IsTriangle{});
+    Scratch scan(s);
+    size_t scan_bytes = 0;
+    e = cub::DeviceScan::InclusiveSum(nullptr, scan_bytes, flags, (uint32_t*)nullptr, n, s);
+    if (e == cudaSuccess) e = scan.reserve(pool, Scratch::pad((size_t)n * 4) + Scratch::pad(scan_bytes));
+    if (e != cudaSuccess) return bail(e);
+    uint32_t* pos = scan.get<uint32_t>(n);
+    void* scan_tmp = scan.get<uint8_t>(scan_bytes);
+    uint32_t nt = 0;
+    e = cub::DeviceScan::InclusiveSum(scan_tmp, scan_bytes, flags, pos, n, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&nt, pos + n - 1, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return bail(e);
+    if (nt == 0) return ok();   // no triangles: an empty BVH, as the host path
+    if (nt > (1u << 29)) return fail(TFG_E_INVALID, "tfgTinyBVHConstruirGPU: too many triangles");
+
+    const size_t nn = 2 * (size_t)nt - 1;
+    size_t sort_bytes = 0;
+    e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                        (uint32_t*)nullptr, (uint32_t*)nullptr, (int)nt, 0, 30, s);
+    if (e != cudaSuccess) return bail(e);
+    Scratch sc(s);
+    const size_t sizes[] = {9 * (size_t)nt * 4, (size_t)nt * sizeof(BNode), sizeof(BuildWords), (size_t)nt * 4,
+                            (size_t)nt * 4, (size_t)nt * 4, (size_t)nt * 4, (size_t)nt * sizeof(int2), nn * 4,
+                            nn * sizeof(BNode), (size_t)nt * sizeof(Plan2), (size_t)nt * 4,
+                            ((size_t)nt + 1) * sizeof(int2), ((size_t)nt + 1) * sizeof(int2),
+                            80 * ((size_t)nt + 1), (size_t)nt * 4, sort_bytes};
+    size_t total = 0;
+    for (size_t b : sizes) total += Scratch::pad(b);
+    e = sc.reserve(pool, total);
+    if (e != cudaSuccess) return bail(e);
     float* verts = sc.get<float>(9 * (size_t)nt);
-    Box6* tbox = sc.get<Box6>(nt);
-    uint32_t* cb = sc.get<uint32_t>(6);
+    BNode* tbox = sc.get<BNode>(nt);
+    BuildWords* words = sc.get<BuildWords>(1);
     uint32_t* code = sc.get<uint32_t>(nt);
     uint32_t* code_s = sc.get<uint32_t>(nt);
     uint32_t* idx = sc.get<uint32_t>(nt);
     uint32_t* idx_s = sc.get<uint32_t>(nt);
-    const uint32_t nn = 2 * nt - 1;
-    int* child = sc.get<int>(2 * (size_t)nt);
+    int2* child = sc.get<int2>(nt);
     int* parent = sc.get<int>(nn);
-    Box6* box = sc.get<Box6>(nn);
-    int* count = sc.get<int>(nn);
-    Plan2* plan = sc.get<Plan2>(nn);
+    BNode* box = sc.get<BNode>(nn);
+    Plan2* plan = sc.get<Plan2>(nt);
     uint32_t* arrivals = sc.get<uint32_t>(nt);
-    int2* q[2] = {sc.get<int2>(nt + 1), sc.get<int2>(nt + 1)};
-    uint32_t* ctr = sc.get<uint32_t>(3);   // next_node, next_tri, queue length
+    int2* q[2];
+    q[0] = sc.get<int2>((size_t)nt + 1);
+    q[1] = sc.get<int2>((size_t)nt + 1);
     uint32_t* nodes = sc.get<uint32_t>(20 * ((size_t)nt + 1));
     uint32_t* tri_order = sc.get<uint32_t>(nt);
-    if (sc.err != cudaSuccess) return bail(sc.err);
-
-    const uint32_t tb = std::min<uint32_t>((nt + 255) / 256, 148u * 8u);
-    k_compact<<<blocks, 256, 0, s>>>(d_prims, n, flag, pos, tris, verts, tbox);
-    const uint32_t init_cb[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
-    e = cudaMemcpyAsync(cb, init_cb, sizeof(init_cb), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return bail(e);
-    k_centroid_bounds<<<tb, 256, 0, s>>>(tbox, nt, cb);
-    k_morton<<<tb, 256, 0, s>>>(tbox, nt, cb, code, idx);
-    size_t sort_bytes = 0;
-    e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, code, code_s, idx, idx_s, (int)nt, 0, 30, s);
-    if (e != cudaSuccess) return bail(e);
     void* sort_tmp = sc.get<uint8_t>(sort_bytes);
-    if (sc.err != cudaSuccess) return bail(sc.err);
+
+    const uint32_t blocks = std::min<uint32_t>(((uint32_t)n + 255) / 256, 148u * 8u);
+    const uint32_t tb = std::min<uint32_t>((nt + 255) / 256, 148u * 8u);
+    k_build_init<<<tb, 256, 0, s>>>(words, q[0], arrivals, nt);
+    k_compact<<<blocks, 256, 0, s>>>(d_prims, n, pos, verts, tbox, words);
+    k_morton<<<tb, 256, 0, s>>>(tbox, nt, words, code, idx);
     e = cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, code, code_s, idx, idx_s, (int)nt, 0, 30, s);
     if (e != cudaSuccess) return bail(e);
-    if (nt > 1) {
-        k_radix_tree<<<tb, 256, 0, s>>>(code_s, (int)nt, child, parent);
-        e = cudaMemsetAsync(arrivals, 0, (size_t)nt * sizeof(uint32_t), s);
-        if (e != cudaSuccess) return bail(e);
-    }
-    k_refit<<<tb, 256, 0, s>>>(tbox, idx_s, (int)nt, child, parent, box, count, plan, arrivals);
-    // Level-by-level collapse; the root is binary node 0 (or the single leaf).
-    const int2 r0 = make_int2(0, 0);   // binary node 0: the root (with one triangle, its leaf)
-    const uint32_t init_ctr[3] = {1u, 0u, 0u};
-    e = cudaMemcpyAsync(q[0], &r0, sizeof(r0), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ctr, init_ctr, sizeof(init_ctr), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return bail(e);
-    uint32_t qn = 1, depth = 0;
-    while (qn > 0) {
-        ++depth;
-        if (depth > 64) {   // a valid tree is far shallower
-            tfgTinyBVHLiberar(out);
-            return fail(TFG_E_BUILD, "tfgTinyBVHConstruirGPU: tree deeper than 64 levels");
+    if (nt > 1) k_radix_tree<<<tb, 256, 0, s>>>(code_s, (int)nt, child, parent);
+    k_refit<<<tb, 256, 0, s>>>(tbox, idx_s, (int)nt, child, parent, box, plan, arrivals);
+    // Level-by-level collapse, kLevelBatch levels per host read.
+    constexpr int kLevelBatch = 8;
+    BuildWords hw;
+    WideArgs wa;
+    wa.child = child; wa.box = box; wa.plan = plan; wa.sorted = idx_s; wa.n = (int)nt;
+    wa.words = words; wa.nodes = nodes; wa.tri_order = tri_order;
+    const uint32_t per_block = kWideThreads / 8;
+    const uint32_t wb = std::min<uint32_t>((nt + per_block - 1) / per_block, 148u * 8u);
+    const size_t pb = Scratch::pad((size_t)nt * sizeof(TfgPrimitiva)), rb = Scratch::pad((size_t)nt * 64),
+                 wtb = Scratch::pad((size_t)nt * 48), node_room = nt / 8 + 16;
+    uint8_t* block = nullptr;
+    int depth = 0;
+    do {
+        for (int k = 0; k < kLevelBatch; ++k, ++depth) {
+            wa.level = depth; wa.q_in = q[depth & 1]; wa.q_out = q[(depth + 1) & 1];
+            k_wide_level<<<wb, kWideThreads, 0, s>>>(wa);
         }
-        WideArgs wa;
-        wa.child = child; wa.box = box; wa.count = count; wa.plan = plan; wa.sorted = idx_s; wa.n = (int)nt;
-        wa.q_in = q[(depth - 1) & 1]; wa.q_n = qn; wa.q_out = q[depth & 1]; wa.q_out_n = ctr + 2;
-        wa.next_node = ctr; wa.next_tri = ctr + 1; wa.nodes = nodes; wa.tri_order = tri_order;
-        e = cudaMemsetAsync(ctr + 2, 0, 4, s);
-        if (e != cudaSuccess) return bail(e);
-        k_wide_level<<<(qn + 127) / 128, 128, 0, s>>>(wa);
-        e = cudaMemcpyAsync(&qn, ctr + 2, 4, cudaMemcpyDeviceToHost, s);
+        if (!block) {
+            // The result, one allocation, made while the GPU works: the
+            // triangle arrays and room for the nodes (trees take 0.11 nodes
+            // per triangle; one that needs more gets them on their own).
+            e = cudaMalloc((void**)&block, pb + rb + wtb + node_room * 80);
+            if (e != cudaSuccess) return bail(e);
+            out->d_primitivas = reinterpret_cast<TfgPrimitiva*>(block);
+            out->num_primitivas = nt;
+            out->ref.d_tris = reinterpret_cast<float*>(block + pb);
+            out->d_tris_wt = reinterpret_cast<float*>(block + pb + rb);
+            bvh_register_block(block);
+        }
+        e = cudaMemcpyAsync(&hw, words, sizeof(hw), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return bail(e);
+    } while (hw.level[depth] != 0 && depth < 64);
+    while (depth > 0 && hw.level[depth - 1] == 0) --depth;
+    if (hw.level[64] != 0) {   // a valid tree is far shallower
+        tfgTinyBVHLiberar(out);
+        return fail(TFG_E_BUILD, "tfgTinyBVHConstruirGPU: tree deeper than 64 levels");
     }
-    uint32_t counts[2] = {0, 0};
-    e = cudaMemcpy(counts, ctr, sizeof(counts), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return bail(e);
-    if (counts[1] != nt) {
+    if (hw.next_tri != nt) {
         tfgTinyBVHLiberar(out);
         return fail(TFG_E_BUILD, "tfgTinyBVHConstruirGPU: leaves do not cover every triangle");
     }
-    const uint32_t num_nodes = counts[0];
-    e = cudaMalloc((void**)&out->ref.d_nodos, (size_t)num_nodes * 80);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&out->ref.d_tris, (size_t)nt * 64);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&out->d_tris_wt, (size_t)nt * 48);
+    const uint32_t num_nodes = hw.next_node;
+    k_emit_tris<<<tb, 256, 0, s>>>(verts, tri_order, nt, out->ref.d_tris, out->d_tris_wt);
+    k_copy_prims<<<blocks, 256, 0, s>>>(d_prims, n, pos, out->d_primitivas);
+    if (num_nodes <= node_room) out->ref.d_nodos = reinterpret_cast<float*>(block + pb + rb + wtb);
+    else e = cudaMalloc((void**)&out->ref.d_nodos, (size_t)num_nodes * 80);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(out->ref.d_nodos, nodes, (size_t)num_nodes * 80, cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return bail(e);
-    k_emit_tris<<<tb, 256, 0, s>>>(verts, tri_order, nt, reinterpret_cast<float*>(out->ref.d_tris), out->d_tris_wt);
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return bail(e);
     out->ref.num_nodos = num_nodes;
     out->ref.num_tris = nt;
-    out->max_depth = depth;
+    out->max_depth = (uint32_t)depth;
     return ok();
 }

@@ -86,6 +86,10 @@ int render_tuning_check(const TfgRenderTuning& t);
 int render_tuning_set(int dev, const TfgRenderTuning& t);
 int render_tuning_get(int dev, TfgRenderTuning* out, uint32_t* generation);
 
+// A device build's result is one allocation starting at `prims`;
+// tfgTinyBVHLiberar frees it as such.
+void bvh_register_block(const void* prims);
+
 int trace_rays(const TfgTinyBVHD_GPU* bvh, const float* tris_wt, int fmt, const float* rays, int n, float* hits,
                cudaStream_t stream);
 
