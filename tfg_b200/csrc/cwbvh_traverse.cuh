@@ -280,6 +280,117 @@ struct CwbvhRay {
     }
 };
 
+// Eight lanes per ray, for queues too short to give every lane a ray of its
+// own: there a launch lasts as long as its slowest ray, and a ray's step is
+// one lane's chain of 48 plane tests.  Here lane j of a group tests the child
+// that comes j-th in the ray's octant order, so the ballot of the hits is the
+// node group as it stands, and a leaf's lane tests its triangles.  The group
+// keeps one traversal state (the same in all its lanes) in a CwbvhRay and its
+// stack in a shared-memory column `st` of kStackTotal entries, `stride` apart.
+// Nodes are visited in the order of one lane's traversal; of a node's
+// triangles the nearest accepted one is kept, the one that is tested first
+// (the highest bit) among equals, which is what testing them in turn keeps.
+// All 32 lanes call this together; `act`: the lane's group has a ray.
+template <int TRI_FMT, bool ANY_HIT>
+__device__ __forceinline__ void group_traverse(CwbvhRay<TRI_FMT, ANY_HIT>& r, bool act, const float4* __restrict__ nodes,
+                                               const float4* __restrict__ tris, uint2* st, int stride) {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, j = lane & 7u, g0 = lane & 24u;
+    while (__any_sync(kFull, act)) {
+        uint32_t tbits = 0, tbase = 0, hit_inner = 0;
+        uint2 ng = r.ng;
+        if (act) {
+            ++r.nsteps;
+            const uint32_t bit = msb_index(ng.y);
+            const uint32_t imask_parent = ng.y & 0xFFu;
+            ng.y &= ~(1u << bit);
+            if (ng.y > 0x00FFFFFFu && r.sp < (uint32_t)kStackTotal) {
+                if (j == 0u) st[r.sp * stride] = ng;
+                ++r.sp;
+            }
+            const uint32_t rel = __popc(imask_parent & ~(kFull << ((bit - 24u) ^ r.octinv)));
+            const float4* node = nodes + 5 * (size_t)(ng.x + rel);
+            const uint8_t* b = reinterpret_cast<const uint8_t*>(node) + (j ^ r.octinv);
+            const float4 n0 = __ldg(node);
+            const uint2 base = __ldg(reinterpret_cast<const uint2*>(node + 1));
+            const uint32_t m = __ldg(b + 24);
+            const uint32_t lx = __ldg(b + 32), ly = __ldg(b + 40), lz = __ldg(b + 48);
+            const uint32_t hx = __ldg(b + 56), hy = __ldg(b + 64), hz = __ldg(b + 72);
+            const uint32_t ew = __float_as_uint(n0.w);
+            const float sx = __uint_as_float((uint32_t)((int)(int8_t)(ew & 0xFF) + 127) << 23);
+            const float sy = __uint_as_float((uint32_t)((int)(int8_t)((ew >> 8) & 0xFF) + 127) << 23);
+            const float sz = __uint_as_float((uint32_t)((int)(int8_t)((ew >> 16) & 0xFF) + 127) << 23);
+            const float idx = sx * r.rD.x, idy = sy * r.rD.y, idz = sz * r.rD.z;
+            const float ox = (n0.x - r.O.x) * r.rD.x, oy = (n0.y - r.O.y) * r.rD.y, oz = (n0.z - r.O.z) * r.rD.z;
+            const bool nx = r.rD.x < 0.0f, ny = r.rD.y < 0.0f, nz = r.rD.z < 0.0f;
+            const float tn = fmaxf(fmaxf(fmaxf(fmaf((float)(nx ? hx : lx), idx, ox), fmaf((float)(ny ? hy : ly), idy, oy)),
+                                         fmaf((float)(nz ? hz : lz), idz, oz)), 0.0f);
+            const float tf = fminf(fminf(fminf(fmaf((float)(nx ? lx : hx), idx, ox), fmaf((float)(ny ? ly : hy), idy, oy)),
+                                         fmaf((float)(nz ? lz : hz), idz, oz)), r.tmax);
+            const bool inner = (m & (m << 1) & 0x10u) != 0u;
+            if (tn <= tf) {
+                hit_inner = inner ? 1u : 0u;
+                if (!inner) tbits = (m >> 5) << (m & 31u);
+            }
+            tbase = base.y;
+            ng = make_uint2(base.x, ew >> 24);
+        }
+        const uint32_t hits = __ballot_sync(kFull, hit_inner != 0u);
+        if (act) r.ng = make_uint2(ng.x, (((hits >> g0) & 0xFFu) << 24) | ng.y);
+        if (__any_sync(kFull, tbits != 0u)) {
+            // this lane's triangles, highest bit first
+            float lt = r.tmax, lu = 0.0f, lv = 0.0f;
+            uint32_t lid = 0;
+            int lk = -1;
+            while (tbits) {
+                const uint32_t k = msb_index(tbits);
+                tbits &= ~(1u << k);
+                float t, u, v;
+                if (TRI_FMT == 0) {
+                    uint32_t tid;
+                    if (!ref_hit(tris, tbase + 4u * k, r.O, r.D, r.tmin, lt, t, u, v, tid)) continue;
+                    lid = tid;
+                } else {
+                    const uint32_t tri = (tbase >> 2) + k;
+                    if (!wt_hit(tris, tri, r.O, r.wr, r.tmin, lt, t, u, v)) continue;
+                    lid = __float_as_uint(__ldg(&tris[3 * tri]).w);
+                }
+                lt = t; lu = u; lv = v; lk = (int)k;
+                if (ANY_HIT) break;
+            }
+            __syncwarp();
+            const uint32_t found = __ballot_sync(kFull, lk >= 0);
+            if (found) {
+                if (ANY_HIT) {
+                    if ((found >> g0) & 0xFFu) { r.found = true; act = false; }
+                } else {
+                    int src = (int)lane;
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) {
+                        const float ot = __shfl_xor_sync(kFull, lt, o);
+                        const int ok = __shfl_xor_sync(kFull, lk, o), os = __shfl_xor_sync(kFull, src, o);
+                        if (ok >= 0 && (lk < 0 || ot < lt || (ot == lt && ok > lk))) { lt = ot; lk = ok; src = os; }
+                    }
+                    lu = __shfl_sync(kFull, lu, src);
+                    lv = __shfl_sync(kFull, lv, src);
+                    lid = __shfl_sync(kFull, lid, src);
+                    if (lk >= 0) { r.tmax = lt; r.hu = lu; r.hv = lv; r.id = lid; r.found = true; }
+                }
+            }
+        }
+        __syncwarp();   // this step's push, before a pop
+        if (act && r.ng.y <= 0x00FFFFFFu) {
+            if (r.sp == 0u) {
+                act = false;
+            } else {
+                --r.sp;
+                r.ng = st[r.sp * stride];
+            }
+        }
+        if (r.nsteps >= kMaxNodeVisits) act = false;
+    }
+}
+
 // Whole traversal in one call.  tmax in: upper bound (exclusive); out: hit
 // distance when found.  Returns true on a hit; id / u / v are written only
 // then.  `cnt`, when not null, accumulates the work done.

@@ -139,16 +139,28 @@ __device__ __forceinline__ void aprim_load(const TfgPrimitiva& p, APrim& q) {
     }
 }
 
+// Products and sums of the analytic tests, each fused or rounded as written,
+// so that every kernel that tests a primitive -- one ray per lane or eight
+// lanes per ray -- finds the same distance to the last bit, whatever the
+// compiler fuses around it.
+__device__ __forceinline__ float dot_fma(V3 a, V3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ V3 cross_fma(V3 a, V3 b) {
+    return v3(__fmaf_rn(a.y, b.z, -__fmul_rn(a.z, b.y)), __fmaf_rn(a.z, b.x, -__fmul_rn(a.x, b.z)),
+              __fmaf_rn(a.x, b.y, -__fmul_rn(a.y, b.x)));
+}
+
 // primitiva.h:121-200: sphere (nearer root above 1e-6), plane (|denom| > 1e-6),
 // Moller-Trumbore triangle (|det| >= 1e-6, t > 1e-6).  u,v = weights of v1,v2.
 __device__ __forceinline__ bool aprim_hit(const APrim& q, V3 O, V3 D, float& t, float& u, float& v) {
     u = 0.0f; v = 0.0f;
     if (q.tipo == TFG_ESFERA) {
         V3 oc = O - v3(q.a[0], q.a[1], q.a[2]);
-        float a = dot(D, D);
-        float b = 2.0f * dot(oc, D);
-        float c = dot(oc, oc) - q.a[3] * q.a[3];
-        float disc = b * b - 4.0f * a * c;
+        float a = dot_fma(D, D);
+        float b = __fmul_rn(2.0f, dot_fma(oc, D));
+        float c = __fmaf_rn(-q.a[3], q.a[3], dot_fma(oc, oc));
+        float disc = __fmaf_rn(b, b, -__fmul_rn(__fmul_rn(4.0f, a), c));
         if (disc < 0.0f) return false;
         float sd = sqrtf(disc);
         float t1 = (-b - sd) / (2.0f * a);
@@ -158,10 +170,10 @@ __device__ __forceinline__ bool aprim_hit(const APrim& q, V3 O, V3 D, float& t, 
         return false;
     } else if (q.tipo == TFG_PLANO) {
         V3 n = v3(q.a[0], q.a[1], q.a[2]);
-        float denom = dot(n, D);
+        float denom = dot_fma(n, D);
         if (fabsf(denom) > 1e-6f) {
-            V3 p0 = n * q.a[3];
-            t = dot(p0 - O, n) / denom;
+            V3 p0 = v3(__fmaf_rn(n.x, q.a[3], -O.x), __fmaf_rn(n.y, q.a[3], -O.y), __fmaf_rn(n.z, q.a[3], -O.z));
+            t = dot_fma(p0, n) / denom;
             return t > 1e-6f;
         }
         return false;
@@ -169,17 +181,17 @@ __device__ __forceinline__ bool aprim_hit(const APrim& q, V3 O, V3 D, float& t, 
         V3 v0 = v3(q.a[0], q.a[1], q.a[2]);
         V3 e1 = v3(q.a[3], q.a[4], q.a[5]) - v0;
         V3 e2 = v3(q.a[6], q.a[7], q.a[8]) - v0;
-        V3 pv = cross(D, e2);
-        float det = dot(e1, pv);
+        V3 pv = cross_fma(D, e2);
+        float det = dot_fma(e1, pv);
         if (fabsf(det) < 1e-6f) return false;
         float inv = 1.0f / det;
         V3 tv = O - v0;
-        u = dot(tv, pv) * inv;
+        u = __fmul_rn(dot_fma(tv, pv), inv);
         if (u < 0.0f || u > 1.0f) return false;
-        V3 qv = cross(tv, e1);
-        v = dot(D, qv) * inv;
-        if (v < 0.0f || u + v > 1.0f) return false;
-        t = dot(e2, qv) * inv;
+        V3 qv = cross_fma(tv, e1);
+        v = __fmul_rn(dot_fma(D, qv), inv);
+        if (v < 0.0f || __fadd_rn(u, v) > 1.0f) return false;
+        t = __fmul_rn(dot_fma(e2, qv), inv);
         return t > 1e-6f;
     }
     return false;

@@ -108,6 +108,7 @@ struct PassArgs {
     int refill_min;           // idle lanes that trigger a traversal warp's refill
     int refill_primary;       // the same for the first bounce
     int shadow_one_lane;      // 1: one lane traces all lights of a shading point
+    uint32_t few_max;         // queues up to this many groups of eight lanes are left to k_few (0: it does not run)
     Workspace ws;
 };
 
@@ -248,6 +249,49 @@ __device__ __forceinline__ bool analytic_any(const APrim* sp, int nsm, const Tfg
     return false;
 }
 
+// The same with eight lanes per ray (all 32 lanes call it together; the
+// result in all lanes of a group): each lane tests every eighth primitive,
+// and the nearest hit, the first primitive's among equals, is what testing
+// them in turn keeps.
+__device__ __forceinline__ int group_analytic_closest(const APrim* sp, int nsm, const TfgPrimitiva* gp, int n, V3 O, V3 D,
+                                                      float& best, float& bu, float& bv) {
+    const int lane = (int)(threadIdx.x & 31u);
+    int hit = n;
+    for (int i = lane & 7; i < n; i += 8) {
+        APrim q;
+        if (i < nsm) q = sp[i];
+        else aprim_load(gp[i], q);
+        float t, u, v;
+        if (aprim_hit(q, O, D, t, u, v) && t < best && t > 1e-6f) { best = t; bu = u; bv = v; hit = i; }
+    }
+    __syncwarp();
+    int src = lane;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const float ot = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+        const int oh = __shfl_xor_sync(0xFFFFFFFFu, hit, o), os = __shfl_xor_sync(0xFFFFFFFFu, src, o);
+        if (oh < n && (hit == n || ot < best || (ot == best && oh < hit))) { best = ot; hit = oh; src = os; }
+    }
+    bu = __shfl_sync(0xFFFFFFFFu, bu, src);
+    bv = __shfl_sync(0xFFFFFFFFu, bv, src);
+    return hit < n ? hit : -1;
+}
+
+__device__ __forceinline__ bool group_analytic_any(const APrim* sp, int nsm, const TfgPrimitiva* gp, int n, V3 O, V3 D,
+                                                   float dist) {
+    const uint32_t lane = threadIdx.x & 31u;
+    bool any = false;
+    for (int i = (int)(lane & 7u); i < n && !any; i += 8) {
+        APrim q;
+        if (i < nsm) q = sp[i];
+        else aprim_load(gp[i], q);
+        float t, u, v;
+        any = aprim_hit(q, O, D, t, u, v) && t > 1e-6f && t < dist;
+    }
+    __syncwarp();
+    return ((__ballot_sync(0xFFFFFFFFu, any) >> (lane & 24u)) & 0xFFu) != 0u;
+}
+
 __device__ __forceinline__ int load_aprims_smem(APrim* sp, const TfgPrimitiva* gp, int n) {
     const int nsm = min(n, kSmemPrims);
     for (int i = threadIdx.x; i < nsm; i += blockDim.x) aprim_load(gp[i], sp[i]);
@@ -327,7 +371,7 @@ __global__ void k_generate(PassArgs a, TableOf<MS> tab) {
 
 // ------------------------------------------------------------------ trace
 template <int TRI_FMT, bool STATS, bool MS>
-__global__ void __launch_bounds__(256) k_trace(PassArgs a, int bounce, TableOf<MS> tab) {
+__global__ void __launch_bounds__(256, MS && !STATS ? 4 : 0) k_trace(PassArgs a, int bounce, TableOf<MS> tab) {
     extern __shared__ unsigned char smem_raw[];
     uint2* sstack = reinterpret_cast<uint2*>(smem_raw);
     APrim* sprims = reinterpret_cast<APrim*>(smem_raw + sizeof(uint2) * kSmemStack * blockDim.x);
@@ -338,6 +382,7 @@ __global__ void __launch_bounds__(256) k_trace(PassArgs a, int bounce, TableOf<M
     st.smem = sstack; st.stride = blockDim.x; st.tid = threadIdx.x;
     const float4* rays = a.ws.ray[bounce & 1];
     const uint32_t n = a.ws.counters[4 * bounce + 0];
+    if (n <= a.few_max) return;
     uint32_t* fetch = &a.ws.counters[4 * bounce + 1];
     TravCounts cnt;
     uint32_t nrays = 0;
@@ -644,17 +689,17 @@ __device__ __forceinline__ bool light_ray(const TfgLuzPuntual& lz, V3 P, V3 N, V
 
 // The shading point's radiance (throughput x light sum) into the path's
 // prefix and / or suffix radiance (dest bit 0: suffix; not 1: prefix too).
-__device__ __forceinline__ void add_direct(const PassArgs& a, uint32_t p, uint32_t dest, V3 cam, V3 L) {
+__device__ __forceinline__ void add_direct(float4* lsuf, float4* lpre, uint32_t p, uint32_t dest, V3 cam, V3 L) {
     const V3 add = mul(cam, L);
     if (dest & 1u) {
-        float4 v = a.ws.lsuf[p];
+        float4 v = lsuf[p];
         v.x += add.x; v.y += add.y; v.z += add.z;
-        a.ws.lsuf[p] = v;
+        lsuf[p] = v;
     }
     if (dest != 1u) {
-        float4 v = a.ws.lpre[p];
+        float4 v = lpre[p];
         v.x += add.x; v.y += add.y; v.z += add.z;
-        a.ws.lpre[p] = v;
+        lpre[p] = v;
     }
 }
 
@@ -666,8 +711,14 @@ __device__ __forceinline__ float4 ld_item(const float4* p) {
     return v;
 }
 
+// Shadow rays of a shading point that k_few runs side by side in a warp.
+template <bool MS>
+__device__ __forceinline__ uint32_t few_rays_per_point(int nl) {
+    return MS || nl <= 1 ? 1u : nl <= 2 ? 2u : 4u;
+}
+
 template <int TRI_FMT, bool STATS, bool MS>
-__global__ void __launch_bounds__(256) k_shadow(PassArgs a, int bounce, TableOf<MS> tab) {
+__global__ void __launch_bounds__(256, (MS || TRI_FMT == 0) && !STATS ? 4 : 0) k_shadow(PassArgs a, int bounce, TableOf<MS> tab) {
     extern __shared__ unsigned char smem_raw[];
     uint2* sstack = reinterpret_cast<uint2*>(smem_raw);
     APrim* sprims = reinterpret_cast<APrim*>(smem_raw + sizeof(uint2) * kSmemStack * blockDim.x);
@@ -675,6 +726,7 @@ __global__ void __launch_bounds__(256) k_shadow(PassArgs a, int bounce, TableOf<
     TravStack stck;
     stck.smem = sstack; stck.stride = blockDim.x; stck.tid = threadIdx.x;
     const uint32_t n = a.ws.counters[4 * bounce + 2];
+    if (n * few_rays_per_point<MS>(a.nlights) <= a.few_max) return;
     uint32_t* fetch = &a.ws.counters[4 * bounce + 3];
     TravCounts cnt;
     uint32_t nrays = 0;
@@ -738,10 +790,109 @@ __global__ void __launch_bounds__(256) k_shadow(PassArgs a, int bounce, TableOf<
         }
         if (have && lg == 0u) {
             const float4 s0 = ld_item(s), s1 = ld_item(s + 1), s3 = ld_item(s + 3);
-            add_direct(a, __float_as_uint(s0.w), __float_as_uint(s1.w), xyz(s3), L);
+            add_direct(a.ws.lsuf, a.ws.lpre, __float_as_uint(s0.w), __float_as_uint(s1.w), xyz(s3), L);
         }
     }
     if (STATS) flush_work(3, nrays, cnt);
+}
+
+// ------------------------------------------------------------------ short queues
+// The closest hits of bounce `tb` and the shadow rays of bounce `sb` (-1:
+// none) when their queues are short, eight lanes per ray (group_traverse).  A
+// traversal launch lasts at least as long as its slowest ray: with one lane
+// per ray that was ~90 us for the 4th to 8th bounce of a 1080p sample, a
+// twentieth of its rays, and 17 us for the 16,384 rays of a 128 x 128 image.
+// All groups take rays first to last and shading points last to first, so
+// that with room for both they run side by side.  `always`: whatever the
+// queues' lengths (a wavefront that starts short); else only what k_trace /
+// k_shadow leave (a.few_max).
+constexpr int kFewThreads = 128;
+
+template <int TRI_FMT, bool MS>
+__global__ void __launch_bounds__(kFewThreads, 8) k_few(PassArgs a, int tb, int sb, int always, TableOf<MS> tab) {
+    __shared__ uint2 sstack[kStackTotal * kFewThreads / 8];
+    __shared__ APrim sprims[MS ? 1 : kSmemPrims];
+    const uint32_t P = few_rays_per_point<MS>(a.nlights);
+    uint32_t n_rays = 0, n_points = 0;
+    if (tb >= 0) {
+        n_rays = a.ws.counters[4 * tb + 0];
+        if (!always && n_rays > a.few_max) n_rays = 0;
+    }
+    if (sb >= 0) {
+        n_points = a.ws.counters[4 * sb + 2];
+        if (!always && n_points * P > a.few_max) n_points = 0;
+    }
+    if (n_rays == 0 && n_points == 0) return;
+    const int nsm = MS ? 0 : load_aprims_smem(sprims, a.prims, a.nprims);
+    Geo g = geo_of<MS>(a, tab, 0);
+    uint2* stack = sstack + threadIdx.x / 8u;
+    constexpr int kStride = kFewThreads / 8;
+    const uint32_t lane = lane_id();
+    const uint32_t groups = gridDim.x * (kFewThreads / 8u), gid = blockIdx.x * (kFewThreads / 8u) + threadIdx.x / 8u;
+    if (n_rays) {
+        const float4* rays = a.ws.ray[tb & 1];
+        for (uint32_t k = gid; __any_sync(0xFFFFFFFFu, k < n_rays); k += groups) {
+            const bool act = k < n_rays;
+            V3 O = v3(0.0f, 0.0f, 0.0f), D = v3(0.0f, 0.0f, 1.0f);
+            float best = 0.0f, bu = 0.0f, bv = 0.0f;
+            if (act) {
+                const float4 o4 = rays[2 * k], d4 = rays[2 * k + 1];
+                O = xyz(o4); D = xyz(d4);
+                if constexpr (MS) { g = geo_of<MS>(a, tab, __float_as_uint(o4.w)); best = 1e9f; }
+                else best = o4.w;
+            }
+            uint32_t bid = kMissId;
+            if (MS || g.nprims > 0) {
+                const int ai = group_analytic_closest(sprims, nsm, g.prims, g.nprims, O, D, best, bu, bv);
+                if (ai >= 0) bid = kAnalyticBit | (uint32_t)ai;
+            }
+            CwbvhRay<TRI_FMT, false> r;
+            r.init(O, D, 0.0f, best);
+            group_traverse(r, act && g.has_bvh, g.nodes, g.tris, stack, kStride);
+            if (r.found && r.tmax < best && r.tmax > kEps) { best = r.tmax; bu = r.hu; bv = r.hv; bid = r.id; }
+            if (act && (lane & 7u) == 0u) a.ws.hit[k] = make_float4(best, bu, bv, __uint_as_float(bid));
+        }
+    }
+    if (n_points) {
+        const uint32_t gw = (31u - lane) / 8u, pl = gw & (P - 1u);   // a point's lights on adjacent groups
+        const uint32_t first = 24u - (gw & ~(P - 1u)) * 8u;          // first lane of its first light's group
+        for (uint32_t i = (groups - 1u - gid) / P; __any_sync(0xFFFFFFFFu, i < n_points); i += groups / P) {
+            const bool have = i < n_points;
+            const float4* s = &a.ws.shadow[4 * (size_t)(have ? i : 0u)];
+            const TfgLuzPuntual* lights = a.lights;
+            int nl = a.nlights;
+            if constexpr (MS) {
+                const uint32_t sc = __float_as_uint(ld_item(s + 2).w);
+                g = geo_of<MS>(a, tab, sc);
+                lights = tab.s[sc].lights; nl = tab.s[sc].nlights;
+            }
+            V3 L = v3(0.0f, 0.0f, 0.0f);
+            for (int l0 = 0; __any_sync(0xFFFFFFFFu, have && l0 < nl); l0 += (int)P) {
+                const int l = l0 + (int)pl;
+                LightRay lr{};
+                bool lit = have && l < nl && light_ray(lights[l], xyz(ld_item(s)), xyz(ld_item(s + 1)), xyz(ld_item(s + 2)), lr);
+                __syncwarp();
+                if (MS || g.nprims > 0) {
+                    if (group_analytic_any(sprims, nsm, g.prims, lit ? g.nprims : 0, lr.so, lr.dl, lr.dist)) lit = false;
+                }
+                CwbvhRay<TRI_FMT, true> r;
+                r.init(lr.so, lr.dl, kEps, lr.dist);
+                group_traverse(r, lit && a.shadow_mesh && g.has_bvh, g.nodes, g.tris, stack, kStride);
+                if (r.found) lit = false;
+                const V3 term = lit ? lr.term : v3(0.0f, 0.0f, 0.0f);
+                for (uint32_t j = 0; j < P; ++j) {   // in light order; an occluded light adds an exact zero
+                    const float x = __shfl_sync(0xFFFFFFFFu, term.x, first - 8u * j);
+                    const float y = __shfl_sync(0xFFFFFFFFu, term.y, first - 8u * j);
+                    const float z = __shfl_sync(0xFFFFFFFFu, term.z, first - 8u * j);
+                    if (l0 + (int)j < nl) L = v3(__fadd_rn(L.x, x), __fadd_rn(L.y, y), __fadd_rn(L.z, z));
+                }
+            }
+            if (have && lane == first) {
+                const float4 s0 = ld_item(s), s1 = ld_item(s + 1), s3 = ld_item(s + 3);
+                add_direct(a.ws.lsuf, a.ws.lpre, __float_as_uint(s0.w), __float_as_uint(s1.w), xyz(s3), L);
+            }
+        }
+    }
 }
 
 // ------------------------------------------------------------------ resolve
@@ -896,6 +1047,7 @@ struct LaunchShapes {
     int trace_occ[2][2][3] = {};
     int shadow_occ[2][2][3] = {};
     int shade_blocks[2] = {0, 0};
+    int few_occ[2][2] = {};          // k_few: [one scene / batch][triangle format]
 };
 LaunchShapes g_shapes[kMaxDevices];
 std::mutex g_shapes_mutex;   // first calls on several host threads fill a device's entry once
@@ -929,6 +1081,10 @@ int shapes_for(int dev, LaunchShapes& s) {
         }
         g.shade_blocks[0] = sms * occ_of(k_shade<false>, 256, 0);
         g.shade_blocks[1] = sms * occ_of(k_shade<true>, 256, 0);
+        g.few_occ[0][0] = occ_of(k_few<0, false>, kFewThreads, 0);
+        g.few_occ[0][1] = occ_of(k_few<1, false>, kFewThreads, 0);
+        g.few_occ[1][0] = occ_of(k_few<0, true>, kFewThreads, 0);
+        g.few_occ[1][1] = occ_of(k_few<1, true>, kFewThreads, 0);
         g.sms = sms;
     }
     s = g;
@@ -1018,6 +1174,11 @@ int pass_workspace(int dev, int slot, uint32_t npix, int spp, bool nrc, cudaStre
     }
     return ensure_workspace(dev, slot, tu.wavefront, nrc, ws);
 }
+
+// Wavefronts up to kFewPaths paths run on k_few alone; longer ones have it
+// beside the long-queue kernels from bounce kFewFrom on.
+constexpr uint32_t kFewPaths = 65536;
+constexpr int kFewFrom = 2;
 
 // Persistent traversal grid: every SM holds as many CTAs as fit, or the
 // tuned number of warps.
@@ -1292,6 +1453,20 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     // same radiance sums, waits for them, so every sum keeps its order.
     const bool overlap = tu.overlap_shadow && ws.side;
     cudaStream_t sstream = overlap ? ws.side : stream;
+    // k_few for short queues: alone, closest hits and the previous bounce's
+    // shadow rays in one launch, for wavefronts that start short; beside the
+    // long-queue kernels from bounce kFewFrom on otherwise (the queue lengths
+    // are only known on the device; a launch with nothing to do takes ~2 us).
+    // Stage timing and work counts keep the stages apart.
+    const uint32_t few_groups = (uint32_t)(sh.sms * sh.few_occ[MS][fmt]) * (kFewThreads / 8u);
+    const bool few_ok = !times && !counts;
+    const uint32_t few_points = MS || a.nlights <= 1 ? 1u : a.nlights <= 2 ? 2u : 4u;   // groups per shading point
+    auto few = [&](int tb, int sb, int always, uint32_t tasks, cudaStream_t st) {
+        const uint32_t fit = (uint32_t)(sh.sms * sh.few_occ[MS][fmt]);
+        const uint32_t grid = std::max(1u, std::min(fit, (tasks + kFewThreads / 8u - 1) / (kFewThreads / 8u)));
+        if (fmt == 0) k_few<0, MS><<<grid, kFewThreads, 0, st>>>(a, tb, sb, always, tab);
+        else k_few<1, MS><<<grid, kFewThreads, 0, st>>>(a, tb, sb, always, tab);
+    };
     a.frame = frame;
     a.img = img;
     a.npix = N;
@@ -1309,8 +1484,21 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
         const int res_blocks = (int)std::max<uint32_t>(1u, std::min<uint32_t>((resolve_n + 255) / 256, (uint32_t)sh.sms * 8u));
         e = cudaMemsetAsync(ws.counters, 0, 4 * (kMaxBounces + 1) * sizeof(uint32_t), stream);
         if (e != cudaSuccess) return fail((int)e, cudaGetErrorString(e));
+        a.few_max = 0;
         stage(0, [&] { k_generate<MS><<<gen_blocks, 256, 0, stream>>>(a, tab); });
+        if (few_ok && a.nq <= kFewPaths) {
+            for (int b = 0; b < prm.max_depth; ++b) {
+                few(b, b - 1, 1, (b == 0 ? 1u : 1u + few_points) * a.nq, stream);
+                k_shade<MS><<<shade_grid, 256, 0, stream>>>(a, b, tab);
+            }
+            few(-1, prm.max_depth - 1, 1, few_points * a.nq, stream);
+            k_resolve<MS><<<res_blocks, 256, 0, stream>>>(a, tab);
+            e = cudaGetLastError();
+            if (e != cudaSuccess) return fail((int)e, std::string("render launch: ") + cudaGetErrorString(e));
+            continue;
+        }
         for (int b = 0; b < prm.max_depth; ++b) {
+            a.few_max = few_ok && b >= kFewFrom ? few_groups : 0u;
             stage(1, [&] {
                 if (fmt == 0) {
                     if (counts) k_trace<0, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
@@ -1319,6 +1507,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
                     if (counts) k_trace<1, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
                     else k_trace<1, false, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
                 }
+                if (a.few_max) few(b, -1, 0, few_groups, stream);
             });
             if (overlap && b > 0) {   // the previous bounce's shadow stage ends before this shade
                 e = cudaStreamWaitEvent(stream, ws.join[b - 1], 0);
@@ -1338,6 +1527,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
                     if (counts) k_shadow<1, true, MS><<<shadow_grid, bt, smem, sstream>>>(a, b, tab);
                     else k_shadow<1, false, MS><<<shadow_grid, bt, smem, sstream>>>(a, b, tab);
                 }
+                if (a.few_max) few(-1, b, 0, few_groups, sstream);
             });
             if (overlap) {
                 e = cudaEventRecord(ws.join[b], sstream);
