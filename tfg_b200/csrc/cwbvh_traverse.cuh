@@ -214,6 +214,11 @@ struct TravCounts {
 // warp are still traversing.  Closest hit (ANY_HIT = false) or first hit
 // (ANY_HIT = true); tmax is the current upper bound (exclusive) and becomes
 // the hit distance; id / hu / hv are valid when `found`.
+//
+// A warp that reconverges between its lanes' node and triangle work calls the
+// turns instead of step(): node_turn() decodes a node and leaves its triangles
+// in tg, tri_turn() tests one of them, next() takes the next node group once
+// tg is empty.  Nodes and triangles come in the same order either way.
 template <int TRI_FMT, bool ANY_HIT>
 struct CwbvhRay {
     V3 O, D, rD;
@@ -222,7 +227,7 @@ struct CwbvhRay {
     float tmin, tmax, hu, hv;
     uint32_t id;
     bool found;
-    uint2 ng;
+    uint2 ng, tg;
     uint32_t sp, nsteps, ntris;
 
     __device__ __forceinline__ void init(V3 O_, V3 D_, float tmin_, float tmax_) {
@@ -231,9 +236,54 @@ struct CwbvhRay {
         octinv = 7u - ((D.x < 0.0f ? 4u : 0u) | (D.y < 0.0f ? 2u : 0u) | (D.z < 0.0f ? 1u : 0u));
         if (TRI_FMT == 1) wr = wt_setup(D);
         ng = make_uint2(0u, 0x80000000u);
+        tg = make_uint2(0u, 0u);
         sp = 0; nsteps = 0; ntris = 0;
         found = false;
         id = 0; hu = 0.0f; hv = 0.0f;
+    }
+
+    __device__ __forceinline__ void node_turn(const float4* __restrict__ nodes, TravStack& st) {
+        ++nsteps;
+        const uint32_t bit = msb_index(ng.y);
+        const uint32_t imask_parent = ng.y & 0xFFu;
+        ng.y &= ~(1u << bit);
+        if (ng.y > 0x00FFFFFFu && sp < (uint32_t)kStackTotal) { st.put(sp, ng); ++sp; }
+        const uint32_t slot = (bit - 24u) ^ octinv;
+        const uint32_t rel = __popc(imask_parent & ~(0xFFFFFFFFu << slot));
+        uint32_t cbase, imask;
+        const uint32_t hm = decode_node(nodes, ng.x + rel, O, rD, octinv, tmax, cbase, tg.x, imask);
+        ng = make_uint2(cbase, (hm & 0xFF000000u) | imask);
+        tg.y = hm & 0x00FFFFFFu;
+    }
+
+    // Tests the highest triangle of tg; true when an any-hit traversal ends.
+    __device__ __forceinline__ bool tri_turn(const float4* __restrict__ tris) {
+        ++ntris;
+        const uint32_t k = msb_index(tg.y);
+        tg.y &= ~(1u << k);
+        float t, u, v;
+        if (TRI_FMT == 0) {
+            uint32_t tid;
+            if (!ref_hit(tris, tg.x + 4u * k, O, D, tmin, tmax, t, u, v, tid)) return false;
+            id = tid;
+        } else {
+            const uint32_t tri = (tg.x >> 2) + k;
+            if (!wt_hit(tris, tri, O, wr, tmin, tmax, t, u, v)) return false;
+            id = __float_as_uint(__ldg(&tris[3 * tri]).w);
+        }
+        tmax = t; hu = u; hv = v; found = true;
+        return ANY_HIT;
+    }
+
+    // Once tg is empty: pops the stack when the node group is, too.  False
+    // when the traversal is complete.
+    __device__ __forceinline__ bool next(TravStack& st) {
+        if (ng.y <= 0x00FFFFFFu) {
+            if (sp == 0) return false;
+            --sp;
+            ng = st.get(sp);
+        }
+        return nsteps < kMaxNodeVisits;
     }
 
     // Decode the next inner node, test its triangles and pop the stack when
