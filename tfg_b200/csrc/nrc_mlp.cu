@@ -488,6 +488,17 @@ __device__ __forceinline__ float scrub(float c) {
     return c;
 }
 
+// A step's kernels are launched with programmatic stream serialisation: a
+// kernel lets the next one start (pdl_launch), and the next one sets itself up
+// and waits for the kernel before it to have finished, its writes visible
+// (pdl_wait).  Two rules keep the chain in order.  A kernel's end implies its
+// predecessors': every block waits before it ends.  And a kernel that touches
+// global memory before its wait, or waits only at its end, starts behind one
+// that calls pdl_launch after its own wait, so that all earlier kernels have
+// finished.  Both calls do nothing in kernels launched the ordinary way.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ bool all_ok(bool ok) { return __syncthreads_and(ok ? 1 : 0) != 0; }
 
 // ------------------------------------------------------------------ inference
@@ -1235,7 +1246,7 @@ struct TrainArgs {
     const uint8_t* bwd;          // BF16 backward image
     uint8_t* hT[kMaxLayers];  // transposed inputs of each layer, per tile
     uint8_t* zT[kMaxLayers];  // transposed output gradients of each layer, per tile
-    float* loss;                 // sum of per-sample losses (unnormalised)
+    float* loss_part;            // per CTA: sum of its per-sample losses (unnormalised)
     uint32_t navail;             // records available when given by the host (written to S_NAVAIL by
                                  // CTA 0 for the later kernels of the step); 0: read S_NAVAIL
     HashGrid hg;                 // composite encoding (levels 0: frequency encoding)
@@ -1309,9 +1320,8 @@ __global__ void __launch_bounds__(kTrainThreads) k_train(TrainArgs a) {
     const int half = t >> 7;                    // columns 32 * half .. 32 * half + 31 of a layer
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t ntiles = a.batch / kTile;
-    const uint32_t n_avail = train_navail(a);
-    const uint32_t seed = a.state[S_STEP];
-    if (blockIdx.x >= ntiles || n_avail < a.min_n || n_avail == 0) return;
+    __shared__ float s_loss[4];
+    pdl_launch();
     if (warp == 0) umma::tmem_alloc(&tslot, 128);
     if (t == 0) {
         umma::mbar_init(&mb_w, 1);
@@ -1326,6 +1336,13 @@ __global__ void __launch_bounds__(kTrainThreads) k_train(TrainArgs a) {
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = tslot;
+    pdl_wait();
+    const uint32_t n_avail = train_navail(a);
+    const uint32_t seed = a.state[S_STEP];
+    if (n_avail < a.min_n || n_avail == 0) {
+        if (warp == 0) umma::tmem_dealloc(tmem, 128);
+        return;
+    }
     if (t == 0) {
         umma::mbar_expect_tx(&mb_w, kFwdBytes<NL> + kBwdBytes<NL>);
         umma::bulk_g2s(sf, a.fwd, kFwdBytes<NL>, &mb_w);
@@ -1464,7 +1481,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_train(TrainArgs a) {
     }
     // loss reduction (the loss lives in the first warpgroup)
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_down_sync(0xFFFFFFFFu, lsum, o);
-    if ((t & 31) == 0 && half == 0) atomicAdd(a.loss, lsum);
+    if ((t & 31) == 0 && half == 0) s_loss[warp] = lsum;
     if (!ok && warp == 0) {   // after a timeout: the weight copy and every issued MMA finish first
         if (umma::elect_one()) {
             if (!weights_in) umma::mbar_wait(&mb_w, 0, kSpinLimit);
@@ -1475,6 +1492,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_train(TrainArgs a) {
     }
     if (!ok && t == 0) atomicExch(&g_mlp_error, 1);
     __syncthreads();
+    if (t == 0) a.loss_part[blockIdx.x] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
     if (warp == 0) umma::tmem_dealloc(tmem, 128);
 }
 
@@ -1499,10 +1517,9 @@ __global__ void __launch_bounds__(128) k_train128(TrainArgs a) {
     __shared__ uint32_t tslot;
     const int t = threadIdx.x, warp = t >> 5;
     const uint32_t ntiles = a.batch / kTile;
-    const uint32_t n_avail = train_navail(a);
-    const uint32_t seed = a.state[S_STEP];
-    if (blockIdx.x >= ntiles || n_avail < a.min_n || n_avail == 0) return;
+    __shared__ float s_loss[4];
     const uint32_t total = (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x * kItems;   // images this CTA loads
+    pdl_launch();
     if (warp == 0) umma::tmem_alloc(&tslot, 256);
     if (t == 0) {
         umma::mbar_init(&mb_w[0], 1);
@@ -1515,6 +1532,13 @@ __global__ void __launch_bounds__(128) k_train128(TrainArgs a) {
     umma::fence_after_sync();
     const uint32_t tmem = tslot;
     const uint32_t tlane = (uint32_t)(32 * warp) << 16;
+    pdl_wait();
+    const uint32_t n_avail = train_navail(a);
+    const uint32_t seed = a.state[S_STEP];
+    if (n_avail < a.min_n || n_avail == 0) {
+        if (warp == 0) umma::tmem_dealloc(tmem, 256);
+        return;
+    }
     // image g % kItems of the per-tile sequence, into buffer g & 1
     bool wpend[2] = {false, false};
     auto load = [&](uint32_t g) {
@@ -1646,7 +1670,7 @@ __global__ void __launch_bounds__(128) k_train128(TrainArgs a) {
         }
     }
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_down_sync(0xFFFFFFFFu, lsum, o);
-    if ((t & 31) == 0) atomicAdd(a.loss, lsum);
+    if ((t & 31) == 0) s_loss[warp] = lsum;
     if (!ok && warp == 0) {   // after a timeout: pending copies and issued MMAs finish first
         if (umma::elect_one()) {
             for (int b = 0; b < 2; ++b)
@@ -1658,6 +1682,7 @@ __global__ void __launch_bounds__(128) k_train128(TrainArgs a) {
     }
     if (!ok && t == 0) atomicExch(&g_mlp_error, 1);
     __syncthreads();
+    if (t == 0) a.loss_part[blockIdx.x] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
     if (warp == 0) umma::tmem_dealloc(tmem, 256);
 }
 
@@ -1823,22 +1848,25 @@ struct WgradArgs {
     uint32_t min_n;
     uint32_t ntiles;
     uint32_t tiles_per_cta;
-    // When set, CTA (0, 0) ends the step (step counter, Adam time, running
-    // loss, as k_tick): the forward / backward kernel that read the step's
-    // seed has finished, and nothing later in a step without hash tables
-    // reads the seed.
+    // The last warp of CTA (0, 0) adds up the step's loss and, when `tick` is
+    // set, ends the step (step counter, Adam time, running loss): every reader
+    // of the step's seed and Adam time but the layers' Adam kernel, which
+    // takes the advanced time, has finished by then.
     int tick;
-    const float* loss_sum;
+    const float* loss_part;      // per-CTA sums of the forward / backward kernel
+    uint32_t loss_ctas;
+    float* loss;
     float inv_count;
+    // The kernel before is the table gradient, which this one runs beside; it
+    // waits for it at its end.
+    int beside;
 };
 
 // Ends a step: advance the step counter and Adam time, keep a running loss.
-__device__ __forceinline__ void tick_state(uint32_t* state, const float* loss_sum, float inv_count, uint32_t min_n) {
-    const uint32_t n = state[S_NAVAIL];
-    if (n < min_n || n == 0) return;
+__device__ __forceinline__ void tick_state(uint32_t* state, float loss_sum, float inv_count) {
     state[S_STEP] += 1u;
     state[S_ADAM_T] += 1u;
-    const float loss = *loss_sum * inv_count;
+    const float loss = loss_sum * inv_count;
     float ema = __uint_as_float(state[S_LOSS_EMA]);
     ema = (state[S_ADAM_T] == 1u) ? loss : 0.9f * ema + 0.1f * loss;
     state[S_LOSS_EMA] = __float_as_uint(ema);
@@ -1855,10 +1883,7 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
     const int l = blockIdx.y;
     const int FZ = l == NL - 1 ? 16 : HID, FH = l == 0 ? 96 : HID;
     const uint32_t t0 = blockIdx.x * a.tiles_per_cta;
-    if (t0 >= a.ntiles || a.state[S_NAVAIL] < a.min_n || a.state[S_NAVAIL] == 0) return;
     const uint32_t t1 = min(a.ntiles, t0 + a.tiles_per_cta);
-    if (a.tick && t == 0 && blockIdx.x == 0 && blockIdx.y == 0)
-        tick_state(const_cast<uint32_t*>(a.state), a.loss_sum, a.inv_count, a.min_n);
     if (warp == 0) umma::tmem_alloc(&tslot, 128);
     if (t == 0) {
         for (int k = 0; k < S; ++k) { umma::mbar_init(&mb_ld[k], 1); umma::mbar_init(&mb_mma[k], 1); }
@@ -1872,6 +1897,14 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = tslot;
+    if (!a.beside) pdl_wait();
+    pdl_launch();   // after the wait: k_adam reads the masters before its own
+    const uint32_t navail = a.state[S_NAVAIL];
+    if (navail < a.min_n || navail == 0) {
+        pdl_wait();
+        if (warp == 0) umma::tmem_dealloc(tmem, 128);
+        return;
+    }
     const uint32_t zbytes = (uint32_t)FZ * 128, hbytes = 2u * FH * 128;
     bool ld_pending[S];
     uint32_t ldph[S], mmph[S];
@@ -1941,6 +1974,17 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
         }
     }
     if (!ok && t == 0) atomicExch(&g_mlp_error, 1);
+    if (a.beside) pdl_wait();
+    if (warp == 3 && blockIdx.x == 0 && blockIdx.y == 0) {
+        float sum = 0.0f;
+        for (uint32_t k = (uint32_t)(t & 31); k < a.loss_ctas; k += 32u) sum += a.loss_part[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        if ((t & 31) == 0) {
+            *a.loss = sum;
+            if (a.tick) tick_state(const_cast<uint32_t*>(a.state), sum, a.inv_count);
+        }
+    }
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, 128);
@@ -1996,26 +2040,33 @@ __device__ __forceinline__ void layer_of(int i, int& l, int& r, int& c) {
 template <int NL, int HID>
 __global__ void k_adam(AdamArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= params_h<HID>(NL)) return;
+    if (i >= params_h<HID>(NL)) { pdl_wait(); return; }
     int l, r, c;
     layer_of<NL, HID>(i, l, r, c);
     // Padded entries (output rows 3..15, input columns past the encoding of layer 0) stay zero.
     const bool live = !(l == NL - 1 && r >= 3) && !(l == 0 && c >= a.live0);
+    // masters, moments and average are this kernel's own: read them while the
+    // gradients are still being formed
     float w = a.w[i];
     float e = a.ema[i];
+    const float m0 = a.m[i], v0 = a.v[i];
+    pdl_wait();
+    pdl_launch();   // after the wait: the tables' Adam kernel waits for this one only at its end
     const bool update = a.update && a.state[S_NAVAIL] >= a.min_n && a.state[S_NAVAIL] > 0;
     const float tn = (float)(a.state[S_ADAM_T] + ((update && !a.ticked) ? 1u : 0u));
     if (update && live) {
         const float bc1 = 1.0f - powf(a.beta1, tn), bc2 = 1.0f - powf(a.beta2, tn);
         float gs = 0.0f;
+#pragma unroll 16
         for (uint32_t k = 0; k < a.groups; ++k) gs += a.part[(size_t)k * params_h<HID>(NL) + i];
         const float g = gs * a.grad_scale;
-        const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * g;
-        const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * g * g;
+        // fused as written, whatever surrounds it: a bit here grows over the steps
+        const float m = __fmaf_rn(1.0f - a.beta1, g, __fmul_rn(a.beta1, m0));
+        const float v = __fmaf_rn(a.beta2, v0, __fmul_rn(__fmul_rn(1.0f - a.beta2, g), g));
         a.m[i] = m;
         a.v[i] = v;
         w -= a.lr * (m / bc1) / (sqrtf(v / bc2) + a.eps);
-        e = a.decay * e + (1.0f - a.decay) * w;
+        e = __fmaf_rn(a.decay, e, __fmul_rn(1.0f - a.decay, w));
         a.w[i] = w;
         a.ema[i] = e;
     }
@@ -2065,6 +2116,8 @@ constexpr int kHashGradSamples = kHashGradThreads / kHashMaxLevels;
 __global__ void __launch_bounds__(kHashGradThreads) k_hash_grad(HashGradArgs a) {
     __shared__ float sw[128][2 * kHashMaxLevels];
     __shared__ float sdz[kHashGradSamples][128 + 1];
+    pdl_wait();
+    pdl_launch();   // after the wait: k_wgrad waits for this kernel only at its end
     const int L2 = 2 * a.hg.levels;
     for (int i = threadIdx.x; i < a.hid * 2 * kHashMaxLevels; i += blockDim.x) {
         const int o = i / (2 * kHashMaxLevels), j = i % (2 * kHashMaxLevels);
@@ -2155,8 +2208,9 @@ struct HashAdamStep {
 // scalar tail.  Gradient, moments, masters and average are read once and
 // written once: 38 bytes per value.
 __global__ void k_adam_hash(HashAdamArgs a) {
+    // (runs beside the layers' Adam kernel, which has waited for both gradients)
     const bool update = a.update && a.state[S_NAVAIL] >= a.min_n && a.state[S_NAVAIL] > 0;
-    const float tn = (float)(a.state[S_ADAM_T] + (update ? 1u : 0u));
+    const float tn = (float)a.state[S_ADAM_T];   // k_wgrad has ended the step
     HashAdamStep st{a.lr, a.beta1, a.beta2, a.eps, a.decay, a.grad_scale,
                     1.0f / (1.0f - powf(a.beta1, tn)), 1.0f / (1.0f - powf(a.beta2, tn)),
                     tn > 0.0f ? 1.0f / (1.0f - powf(a.decay, tn)) : 0.0f, update};
@@ -2187,6 +2241,8 @@ __global__ void k_adam_hash(HashAdamArgs a) {
         a.grad[i] = 0.0f;
         a.infer[i] = __float2half_rn(r);
     }
+    pdl_launch();
+    pdl_wait();
 }
 
 // Initial table values: uniform in (-1e-4, 1e-4) (Mueller et al. 2022),
@@ -2200,13 +2256,6 @@ __global__ void k_hash_init(float* w, size_t count, uint64_t seed) {
         const float u = (float)(z >> 40) * (1.0f / 16777216.0f);
         w[i] = (2.0f * u - 1.0f) * 1e-4f;
     }
-}
-
-// After a step of a model with hash-grid tables (whose table gradient reads
-// the step's seed after k_wgrad): the same end of step as k_wgrad's.
-__global__ void k_tick(uint32_t* state, const float* loss_sum, float inv_count, uint32_t min_n) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    tick_state(state, loss_sum, inv_count, min_n);
 }
 
 // ------------------------------------------------------------------ cache gate
@@ -2301,7 +2350,7 @@ struct ColorMlp {
     int hid = 64;                // hidden width (64 or 128)
     uint8_t* hT[mlp::kMaxLayers] = {nullptr};
     uint8_t* zT[mlp::kMaxLayers] = {nullptr};
-    float* loss = nullptr;
+    float* loss = nullptr;       // the last step's loss sum, then one partial sum per forward / backward CTA
     uint32_t* dstate = nullptr;  // mlp::S_* words
     float gate = 0.0f;           // gate threshold on a cell's relative bias (<= 0: no gate)
     float4* gate_cells = nullptr;   // running sums per gate cell (allocated with the first threshold > 0)
@@ -2386,7 +2435,26 @@ uint64_t splitmix(uint64_t& s) {
     return z ^ (z >> 31);
 }
 
-int repack(ColorMlp* n, cudaStream_t s, bool update, uint32_t min_n, bool ticked) {
+// Launch that may start before the kernel ahead of it in the stream has
+// finished; the kernel itself waits for it (mlp::pdl_wait).
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Adam step of the layers (or, without `update`, their operand images from the
+// masters and average as they are).
+int enqueue_adam(ColorMlp* n, cudaStream_t s, bool update, uint32_t min_n) {
     mlp::AdamArgs a;
     a.w = n->w; a.m = n->m; a.v = n->v; a.ema = n->ema; a.grad = n->grad;
     a.part = update ? n->wpart : nullptr;
@@ -2398,26 +2466,42 @@ int repack(ColorMlp* n, cudaStream_t s, bool update, uint32_t min_n, bool ticked
     a.min_n = min_n;
     a.update = update ? 1 : 0;
     a.live0 = n->hlevels ? mlp::kHashLive : mlp::kFreqLive;
-    a.ticked = ticked ? 1 : 0;
+    a.ticked = update ? 1 : 0;   // k_wgrad has ended the step
+    cudaError_t e = cudaSuccess;
     with_width(n, [&](auto c, auto w) {
         constexpr int NL = decltype(c)::value, HID = decltype(w)::value;
-        mlp::k_adam<NL, HID><<<(mlp::params_h<HID>(NL) + 255) / 256, 256, 0, s>>>(a);
+        const unsigned blocks = (mlp::params_h<HID>(NL) + 255) / 256;
+        if (update) e = launch_early(mlp::k_adam<NL, HID>, dim3(blocks), 256, 0, s, a);
+        else mlp::k_adam<NL, HID><<<blocks, 256, 0, s>>>(a);
         return 0;
     });
-    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "mlp adam");
-    if (n->hlevels) {
-        mlp::HashAdamArgs h;
-        h.w = n->hw; h.m = n->hm; h.v = n->hv; h.ema = n->hema; h.grad = n->hgrad; h.infer = n->hinf;
-        h.count = n->hcount;
-        h.lr = n->lr; h.beta1 = n->beta1; h.beta2 = n->beta2; h.eps = n->eps; h.decay = n->decay;
-        h.grad_scale = a.grad_scale;
-        h.state = n->dstate; h.min_n = min_n; h.update = a.update;
-        mlp::k_adam_hash<<<(unsigned)std::min<size_t>((n->hcount + 255) / 256, (size_t)n->sms * 16), 256, 0, s>>>(h);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_fail(e, "mlp adam (tables)");
-    }
     return ok();
+}
+
+// The same for the hash-grid tables, if the model has any.
+int enqueue_adam_hash(ColorMlp* n, cudaStream_t s, bool update, uint32_t min_n) {
+    if (!n->hlevels) return ok();
+    mlp::HashAdamArgs h;
+    h.w = n->hw; h.m = n->hm; h.v = n->hv; h.ema = n->hema; h.grad = n->hgrad; h.infer = n->hinf;
+    h.count = n->hcount;
+    h.lr = n->lr; h.beta1 = n->beta1; h.beta2 = n->beta2; h.eps = n->eps; h.decay = n->decay;
+    h.grad_scale = 1.0f / (3.0f * (float)n->batch);
+    h.state = n->dstate; h.min_n = min_n; h.update = update ? 1 : 0;
+    const unsigned blocks = (unsigned)std::min<size_t>((n->hcount + 255) / 256, (size_t)n->sms * 16);
+    cudaError_t e = cudaSuccess;
+    if (update) e = launch_early(mlp::k_adam_hash, dim3(blocks), 256, 0, s, h);
+    else mlp::k_adam_hash<<<blocks, 256, 0, s>>>(h);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "mlp adam (tables)");
+    return ok();
+}
+
+// Operand images of parameters that were set or loaded.
+int repack(ColorMlp* n, cudaStream_t s) {
+    if (int rc = enqueue_adam(n, s, false, 1)) return rc;
+    return enqueue_adam_hash(n, s, false, 1);
 }
 
 int ensure_acts(ColorMlp* n, uint32_t tiles) {
@@ -2469,7 +2553,11 @@ uint32_t infer_grid(const ColorMlp* n, uint32_t tiles) {
     return std::max<uint32_t>(1u, std::min<uint32_t>((tiles + mlp::kSlots - 1) / mlp::kSlots, cap));
 }
 
-int enqueue_wgrad(ColorMlp* n, uint32_t tiles_per_cta, uint32_t min_n, cudaStream_t s, bool tick = false) {
+// Weight gradients of the batch the last forward / backward kernel ran.
+// `in_step`: launched early behind the step's previous kernel (the forward /
+// backward kernel, or with `beside` the table gradient that it runs beside).
+int enqueue_wgrad(ColorMlp* n, uint32_t tiles_per_cta, uint32_t min_n, cudaStream_t s, bool in_step = false,
+                  bool beside = false, bool tick = false) {
     const uint32_t tiles = n->batch / mlp::kTile;
     mlp::WgradArgs wa;
     for (int l = 0; l < mlp::kMaxLayers; ++l) { wa.zT[l] = n->zT[l]; wa.hT[l] = n->hT[l]; }
@@ -2477,15 +2565,21 @@ int enqueue_wgrad(ColorMlp* n, uint32_t tiles_per_cta, uint32_t min_n, cudaStrea
     wa.ntiles = tiles;
     wa.tiles_per_cta = std::max<uint32_t>(1u, tiles_per_cta);
     wa.tick = tick ? 1 : 0;
-    wa.loss_sum = n->loss;
+    wa.loss_part = n->loss + 1;
+    wa.loss_ctas = std::min<uint32_t>(tiles, (uint32_t)n->sms);
+    wa.loss = n->loss;
+    wa.beside = beside ? 1 : 0;
     wa.inv_count = 1.0f / (3.0f * (float)n->batch);
     const uint32_t groups = (tiles + wa.tiles_per_cta - 1) / wa.tiles_per_cta;
+    cudaError_t e = cudaSuccess;
     with_width(n, [&](auto c, auto w) {
         constexpr int NL = decltype(c)::value, HID = decltype(w)::value;
-        mlp::k_wgrad<NL, HID><<<dim3(groups, NL), 128, mlp::kWgSmemH<HID> + 1024, s>>>(wa);
+        const size_t sm = mlp::kWgSmemH<HID> + 1024;
+        if (in_step) e = launch_early(mlp::k_wgrad<NL, HID>, dim3(groups, NL), 128, sm, s, wa);
+        else mlp::k_wgrad<NL, HID><<<dim3(groups, NL), 128, sm, s>>>(wa);
         return 0;
     });
-    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "mlp step: weight gradients");
     n->wgroups = groups;
     return ok();
@@ -2511,45 +2605,38 @@ int enqueue_wgrad_sum(ColorMlp* n, uint32_t min_n, cudaStream_t s) {
 int enqueue_step(ColorMlp* n, const TfgDatosMLP* buf, uint32_t min_n, bool update, cudaStream_t s,
                  uint32_t navail = 0) {
     const uint32_t tiles = n->batch / mlp::kTile;
-    cudaError_t e = cudaMemsetAsync(n->loss, 0, sizeof(float), s);
-    if (e != cudaSuccess) return cuda_fail(e, "mlp step");
+    cudaError_t e = cudaSuccess;
     mlp::TrainArgs ta;
     ta.buf = buf; ta.state = n->dstate; ta.min_n = min_n; ta.batch = n->batch;
-    ta.bounds = n->bounds; ta.fwd = n->fwd; ta.bwd = n->bwd; ta.loss = n->loss;
+    ta.bounds = n->bounds; ta.fwd = n->fwd; ta.bwd = n->bwd; ta.loss_part = n->loss + 1;
     ta.hg = hash_view(n, true);
     ta.navail = navail;
     for (int l = 0; l < mlp::kMaxLayers; ++l) { ta.hT[l] = n->hT[l]; ta.zT[l] = n->zT[l]; }
     with_width(n, [&](auto c, auto w) {
         constexpr int NL = decltype(c)::value, HID = decltype(w)::value;
         const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)n->sms);
-        if constexpr (HID == 128) mlp::k_train128<NL><<<grid, 128, mlp::kT128Smem + 1024, s>>>(ta);
-        else mlp::k_train<NL><<<grid, mlp::kTrainThreads, mlp::kTrainSmem + 1024, s>>>(ta);
+        if constexpr (HID == 128) e = launch_early(mlp::k_train128<NL>, dim3(grid), 128, mlp::kT128Smem + 1024, s, ta);
+        else e = launch_early(mlp::k_train<NL>, dim3(grid), mlp::kTrainThreads, mlp::kTrainSmem + 1024, s, ta);
         return 0;
     });
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "mlp step: forward/backward");
-    // Without hash tables the weight-gradient kernel ends the step; the table
-    // gradient re-draws the step's samples from its seed, so with tables
-    // k_tick ends it after the table update.
-    const bool tick_early = update && n->hlevels == 0;
-    if (int rc = enqueue_wgrad(n, wgrad_tiles_per_cta(n, tiles), min_n, s, tick_early)) return rc;
+    // The table gradient (atomics), which re-draws the step's samples from its
+    // seed, runs beside the weight gradients (tensor cores, 96 CTAs), whose
+    // kernel ends the step; then the two Adam kernels run side by side.
     if (n->hlevels) {
         mlp::HashGradArgs ha;
         ha.buf = buf; ha.state = n->dstate; ha.min_n = min_n; ha.batch = n->batch; ha.bounds = n->bounds;
         ha.zT0 = n->zT[0]; ha.w0 = n->w; ha.grad = reinterpret_cast<float2*>(n->hgrad); ha.hg = hash_view(n, true);
         ha.hid = n->hid;
-        mlp::k_hash_grad<<<(n->batch + mlp::kHashGradSamples - 1) / mlp::kHashGradSamples, mlp::kHashGradThreads, 0, s>>>(ha);
-        e = cudaGetLastError();
+        e = launch_early(mlp::k_hash_grad, dim3((n->batch + mlp::kHashGradSamples - 1) / mlp::kHashGradSamples),
+                         mlp::kHashGradThreads, 0, s, ha);
         if (e != cudaSuccess) return cuda_fail(e, "mlp step: table gradient");
     }
+    if (int rc = enqueue_wgrad(n, wgrad_tiles_per_cta(n, tiles), min_n, s, true, n->hlevels != 0, update)) return rc;
     if (!update) return enqueue_wgrad_sum(n, min_n, s);
-    if (int rc = repack(n, s, true, min_n, tick_early)) return rc;
-    if (n->hlevels) {
-        mlp::k_tick<<<1, 32, 0, s>>>(n->dstate, n->loss, 1.0f / (3.0f * (float)n->batch), min_n);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_fail(e, "mlp step: tick");
-    }
-    return ok();
+    if (int rc = enqueue_adam(n, s, true, min_n)) return rc;
+    return enqueue_adam_hash(n, s, true, min_n);
 }
 
 int set_word(ColorMlp* n, int index, uint32_t value, cudaStream_t s) {
@@ -2982,7 +3069,8 @@ int create_model(uint32_t n_in, uint32_t n_out, uint32_t batch, uint64_t seed, i
     if (e == cudaSuccess) e = cudaMalloc((void**)&n->inf_bf, fwd_bytes);
     if (e == cudaSuccess) e = cudaMalloc((void**)&n->inf_f8, f8_bytes);
     if (e == cudaSuccess) e = cudaMalloc((void**)&n->f8, M::kF8Words * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&n->loss, sizeof(float));
+    const size_t loss_bytes = (1 + (size_t)n->sms) * sizeof(float);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&n->loss, loss_bytes);
     if (e == cudaSuccess) e = cudaMalloc((void**)&n->dstate, M::S_WORDS * sizeof(uint32_t));
     if (e != cudaSuccess) { tfgMlpDestroy(reinterpret_cast<TfgColorMLP*>(n)); return tfg::cuda_fail(e, "tfgMlpCreate"); }
     cudaMemset(n->fwd, 0, fwd_bytes);
@@ -2990,6 +3078,7 @@ int create_model(uint32_t n_in, uint32_t n_out, uint32_t batch, uint64_t seed, i
     cudaMemset(n->inf, 0, fwd_bytes);
     cudaMemset(n->inf_bf, 0, fwd_bytes);
     cudaMemset(n->inf_f8, 0, f8_bytes);
+    cudaMemset(n->loss, 0, loss_bytes);
     cudaMemset(n->f8, 0, M::kF8Words * sizeof(float));
     cudaMemset(n->dstate, 0, M::S_WORDS * sizeof(uint32_t));
     if (hc) {
@@ -3017,7 +3106,7 @@ int create_model(uint32_t n_in, uint32_t n_out, uint32_t batch, uint64_t seed, i
     if (e == cudaSuccess) e = cudaMemset(n->v, 0, pb);
     if (e == cudaSuccess) e = cudaMemset(n->grad, 0, pb);
     if (e != cudaSuccess) { tfgMlpDestroy(reinterpret_cast<TfgColorMLP*>(n)); return tfg::cuda_fail(e, "tfgMlpCreate"); }
-    if (int rc = tfg::repack(n, 0, false, 1, false)) { tfgMlpDestroy(reinterpret_cast<TfgColorMLP*>(n)); return rc; }
+    if (int rc = tfg::repack(n, 0)) { tfgMlpDestroy(reinterpret_cast<TfgColorMLP*>(n)); return rc; }
     static bool attrs = false;
     if (!attrs) {
         set_kernel_attrs<4>();
@@ -3310,7 +3399,7 @@ extern "C" int tfgMlpSetParams(TfgColorMLP* h, const float* host, uint32_t count
         if (e == cudaSuccess) e = cudaMemset(n->hgrad, 0, hb);
     }
     if (e != cudaSuccess) return tfg::cuda_fail(e, "tfgMlpSetParams");
-    if (int rc = tfg::repack(n, 0, false, 1, false)) return rc;
+    if (int rc = tfg::repack(n, 0)) return rc;
     e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return tfg::cuda_fail(e, "tfgMlpSetParams");
     return tfg::ok();
@@ -3484,7 +3573,7 @@ extern "C" int tfgMlpLoad(TfgColorMLP* h, const char* path) {
     if (e != cudaSuccess) return tfg::cuda_fail(e, "tfgMlpLoad");
     n->bounds = M::Bounds{{lo[0], lo[1], lo[2]}, {hi[0], hi[1], hi[2]}};
     n->lr = hyper[0]; n->beta1 = hyper[1]; n->beta2 = hyper[2]; n->eps = hyper[3]; n->decay = hyper[4];
-    if (int rc = tfg::repack(n, 0, false, 1, false)) return rc;   // operand images of the loaded arrays
+    if (int rc = tfg::repack(n, 0)) return rc;   // operand images of the loaded arrays
     e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return tfg::cuda_fail(e, "tfgMlpLoad");
     return tfg::ok();
