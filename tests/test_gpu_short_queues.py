@@ -138,3 +138,51 @@ def test_batches_with_short_queues(built, sizes):
         np.testing.assert_array_equal(a, b)
     for d in dss:
         d.close()
+
+
+def test_passes_that_follow_each_other_closely(built):
+    """Kernels of short wavefronts start before their predecessors end: passes
+    back to back, in several wavefronts each, with writes to what they read
+    between them, directly and as a replayed graph."""
+    ds = pt.DeviceScene(scenes.reference_room(64, 48, subdiv=2), "cuda")
+    n = 64 * 48
+    p = pt.RenderParams(max_depth=6, rr_min_depth=3, shadow_mesh=1, spp=2, accumulate=1)
+    imgs = [torch.zeros(n * 3, device="cuda") for _ in range(4)]
+    acc = torch.zeros(n * 3, device="cuda")
+
+    def passes():
+        acc.zero_()
+        for k, img in enumerate(imgs):
+            pt.render_pass(ds, p, 2 * k, img, acc)
+            acc.mul_(0.5)
+
+    want = []
+    for k in range(4):   # one at a time
+        if k == 0:
+            acc.zero_()
+        pt.render_pass(ds, p, 2 * k, imgs[k], acc)
+        torch.cuda.synchronize()
+        acc.mul_(0.5)
+        torch.cuda.synchronize()
+    want = [acc.clone()] + [i.clone() for i in imgs]
+
+    for wavefront in (0, 1024):
+        pt.set_tuning(pt.RenderTuning.default() if not wavefront else pt.RenderTuning(wavefront_paths=wavefront))
+        passes()
+        torch.cuda.synchronize()
+        for a, b in zip([acc] + imgs, want):
+            assert torch.equal(a, b)
+    pt.set_tuning(pt.RenderTuning.default())
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        passes()
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            passes()
+        for _ in range(3):
+            g.replay()
+        s.synchronize()
+    for a, b in zip([acc] + imgs, want):
+        assert torch.equal(a, b)
+    ds.close()
