@@ -40,6 +40,10 @@ WORKLOAD = "plain path tracing, 1920x1080, 64 spp, depth 8, RR from depth 3, 16 
 TRACE_DRAM_BYTES_PER_RAY = {1: 76.57, 16: 63.12}
 
 
+# Wavefronts hold whole samples up to this many paths when the tuning leaves
+# their size open (wavefront_paths 0).
+AUTO_PATHS = 1 << 24
+
 # ncu counters of the closest-hit kernel on the bench frame (one-sample pass,
 # all eight bounces; profiles/k_trace_l2_issue_1080p.md): L2 bytes
 # (lts__t_bytes.sum) per closest-hit ray traced, the share of issue slots
@@ -93,7 +97,7 @@ def trace_traffic(wavefront_paths: int, n_px: int, rays_per_launch: float) -> in
     """DRAM bytes per closest-hit launch: the measured bytes per ray of the
     nearest captured wavefront size (1 or 16 samples) times the rays of an
     average launch."""
-    k = max(1, wavefront_paths // n_px) if wavefront_paths else 1
+    k = max(1, (wavefront_paths or AUTO_PATHS) // n_px)
     return int(round(TRACE_DRAM_BYTES_PER_RAY[1 if k < 4 else 16] * rays_per_launch))
 
 
@@ -1082,7 +1086,7 @@ def main():
         del rays, hits
         return samples * n_px * reps / (p0.elapsed_time(p1) * 1e-3) / 1e9
 
-    primary_samples = max(1, min(16, tuning.wavefront_paths // n_px)) if tuning.wavefront_paths else 1
+    primary_samples = max(1, min(16, (tuning.wavefront_paths or AUTO_PATHS) // n_px))
     primary_grays = primary(primary_samples, pt.RAYS_TILES)
     primary_one = {"scanline": round(primary(1, pt.RAYS_SCANLINE), 3), "tiles": round(primary(1, pt.RAYS_TILES), 3)}
 

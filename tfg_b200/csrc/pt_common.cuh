@@ -202,40 +202,63 @@ struct Material {
     V3 emision, difuso, especular, transmision;
     float ior;
 };
-__device__ __forceinline__ Material load_material(const TfgPrimitiva* p) {
+// A primitive as the shading stage reads it: type, material and vertex normals
+// requested together, in 8-byte loads (the struct's own alignment), so that a
+// hit waits for one gather, not for three in a row (type, normals, material).
+// The vertices, which only flat triangles need, follow.
+struct PrimRow {
+    int tipo;
     Material m;
-    m.emision = ld3(p->emision);
-    m.difuso = ld3(p->difuso);
-    m.especular = ld3(p->especular);
-    m.transmision = ld3(p->transmision);
-    m.ior = p->indice_refraccion;
-    return m;
+    double first[3];          // triangulo.v0 / esfera.centro / plano.normal
+    double normals[9];        // triangulo.v0_normal, v1_normal, v2_normal
+    const double* vertices;   // triangulo.v0, v1, v2, for flat triangles only
+};
+__device__ __forceinline__ PrimRow load_prim(const TfgPrimitiva* p) {
+    static_assert(sizeof(TfgPrimitiva) == 200 && offsetof(TfgPrimitiva, u) == 56, "layout");
+    const uint2* w = reinterpret_cast<const uint2*>(p);
+    const double* d = reinterpret_cast<const double*>(w + 7);
+    PrimRow r;
+    const uint2 a = w[0], b = w[1], c = w[2], e = w[3], f = w[4], g = w[5], h = w[6];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) r.first[i] = d[i];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) r.normals[i] = d[9 + i];
+    r.vertices = d;
+    r.tipo = (int)a.x;
+    r.m.emision = v3(__uint_as_float(a.y), __uint_as_float(b.x), __uint_as_float(b.y));
+    r.m.difuso = v3(__uint_as_float(c.x), __uint_as_float(c.y), __uint_as_float(e.x));
+    r.m.especular = v3(__uint_as_float(e.y), __uint_as_float(f.x), __uint_as_float(f.y));
+    r.m.transmision = v3(__uint_as_float(g.x), __uint_as_float(g.y), __uint_as_float(h.x));
+    r.m.ior = __uint_as_float(h.y);
+    return r;
 }
 
 // escenario.h:123-142 with primitiva.h:84-101 (smooth) and :202-220 (flat):
 // triangles with differing vertex normals are shaded with the barycentric
 // normal, others with the face normal turned toward the world origin; spheres
 // use (p - c)/|p - c|; planes use the stored normal as is (not renormalised).
-__device__ __forceinline__ V3 surface_normal(const TfgPrimitiva* p, V3 P, float u, float v) {
-    if (p->tipo == TFG_TRIANGULO) {
-        const TfgVec3d& n0 = p->u.triangulo.v0_normal;
-        const TfgVec3d& n1 = p->u.triangulo.v1_normal;
-        const TfgVec3d& n2 = p->u.triangulo.v2_normal;
-        bool smooth = (n0.x != n1.x || n0.y != n1.y || n0.z != n1.z) || (n0.x != n2.x || n0.y != n2.y || n0.z != n2.z);
+__device__ __forceinline__ V3 surface_normal(const PrimRow& p, V3 P, float u, float v) {
+    const V3 v0 = v3((float)p.first[0], (float)p.first[1], (float)p.first[2]);
+    if (p.tipo == TFG_TRIANGULO) {
+        const double *n0 = p.normals, *n1 = n0 + 3, *n2 = n0 + 6;
+        bool smooth = (n0[0] != n1[0] || n0[1] != n1[1] || n0[2] != n1[2]) ||
+                      (n0[0] != n2[0] || n0[1] != n2[1] || n0[2] != n2[2]);
         if (smooth) {
             float b0 = 1.0f - u - v;
-            V3 n = ld3(n0) * b0 + ld3(n1) * u + ld3(n2) * v;
+            V3 n = v3((float)n0[0], (float)n0[1], (float)n0[2]) * b0 + v3((float)n1[0], (float)n1[1], (float)n1[2]) * u +
+                   v3((float)n2[0], (float)n2[1], (float)n2[2]) * v;
             float len = sqrtf(dot(n, n));
             if (len > 1e-6f) return n * (1.0f / len);
             return v3(0.0f, 0.0f, 0.0f);
         }
-        V3 a = ld3(p->u.triangulo.v0);
-        V3 n = cross(ld3(p->u.triangulo.v1) - a, ld3(p->u.triangulo.v2) - a);
+        V3 a = v0;
+        const double* w = p.vertices;
+        V3 n = cross(v3((float)w[3], (float)w[4], (float)w[5]) - a, v3((float)w[6], (float)w[7], (float)w[8]) - a);
         if (dot(n, -P) < 0.0f) n = n * -1.0f;
         return normalized(n);
     }
-    if (p->tipo == TFG_ESFERA) return normalized(P - ld3(p->u.esfera.centro));
-    if (p->tipo == TFG_PLANO) return ld3(p->u.plano.normal);
+    if (p.tipo == TFG_ESFERA) return normalized(P - v0);
+    if (p.tipo == TFG_PLANO) return v0;
     return v3(0.0f, 0.0f, 0.0f);
 }
 

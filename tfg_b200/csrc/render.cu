@@ -503,8 +503,18 @@ __device__ __forceinline__ void write_datos(TfgDatosMLP* d, V3 P, V3 dir, V3 n, 
     *d = r;
 }
 
+// Bound by the latency of its gathers (20 warps per SM, forty loads per
+// path, a third of the issue slots and 2.7 TB/s in use), so a path's state and
+// its primitive are requested together (load_prim), and radiance is read and
+// written only where it changes.  Blocks of 128 spread short queues over more
+// SMs and fill the register file better than 256.  With the same in k_resolve
+// (flags read only for the cache): 128 x 128 350 -> 330 us, 16 samples of
+// 1920 x 1080 10.55 -> 10.38 ms.  More warps by a register limit: 6 blocks per
+// SM 10.9 ms, 7 10.9, 8 11.0.
+constexpr int kShadeThreads = 128;
+
 template <bool MS>
-__global__ void __launch_bounds__(256) k_shade(PassArgs a, int bounce, TableOf<MS> tab) {
+__global__ void __launch_bounds__(kShadeThreads) k_shade(PassArgs a, int bounce, TableOf<MS> tab) {
     pdl_sync();
     const uint32_t n = a.ws.counters[4 * bounce + 0];
     const float4* rays = a.ws.ray[bounce & 1];
@@ -536,20 +546,19 @@ __global__ void __launch_bounds__(256) k_shade(PassArgs a, int bounce, TableOf<M
             uint32_t rng = st.x, flags = st.y;
             float pdf_last = __uint_as_float(st.z);
             const uint32_t id = __float_as_uint(h.w);
-            float4 lpre = a.ws.lpre[p];
-            float4 lsuf = make_float4(0, 0, 0, 0), nrc4 = make_float4(0, 0, 0, 0);
-            if (nrc) { lsuf = a.ws.lsuf[p]; nrc4 = a.ws.nrc[p]; }
+            float4 lpre = make_float4(0, 0, 0, 0), lsuf = lpre, nrc4 = lpre;
+            if (nrc) { lpre = a.ws.lpre[p]; lsuf = a.ws.lsuf[p]; nrc4 = a.ws.nrc[p]; }
             bool end = false;
             if (id == kMissId) {
                 end = true;   // background is black (render.h:227-239)
             } else {
-                const TfgPrimitiva* pr = prim_of(g, id);
+                const PrimRow pr = load_prim(prim_of(g, id));
                 const float t = h.x;
                 const V3 P = O + D * t;
                 const V3 nrm = surface_normal(pr, P, h.y, h.z);
                 const V3 view = -D;
                 const float cos_t = fabsf(dot(nrm, -D));
-                const Material m = load_material(pr);
+                const Material& m = pr.m;
                 const bool es_dif = cmax(m.difuso) > kEps;
                 const bool es_esp = cmax(m.especular) > kEps;
                 const bool captured = (flags & F_CAPTURED) != 0;
@@ -577,7 +586,9 @@ __global__ void __launch_bounds__(256) k_shade(PassArgs a, int bounce, TableOf<M
                         a.ws.ts[10 * (size_t)p + 9] = make_float4(0, 0, 0, 0);
                         flags |= F_TAIL;
                     } else {
+                        if (!nrc) lpre = a.ws.lpre[p];
                         lpre.x += c.x; lpre.y += c.y; lpre.z += c.z;
+                        if (!nrc) a.ws.lpre[p] = lpre;
                     }
                     end = true;
                 } else {
@@ -680,8 +691,7 @@ __global__ void __launch_bounds__(256) k_shade(PassArgs a, int bounce, TableOf<M
             }
             a.ws.thr[p] = make_float4(cam.x, cam.y, cam.z, ior);
             a.ws.st[p] = make_uint4(rng, flags, __float_as_uint(pdf_last), st.w);
-            a.ws.lpre[p] = lpre;
-            if (nrc) { a.ws.lsuf[p] = lsuf; a.ws.nrc[p] = nrc4; }
+            if (nrc) { a.ws.lpre[p] = lpre; a.ws.lsuf[p] = lsuf; a.ws.nrc[p] = nrc4; }
             nr0 = make_float4(O.x, O.y, O.z, MS ? __uint_as_float(sc) : 1e9f);
             nr1 = make_float4(D.x, D.y, D.z, __uint_as_float(p));
         }
@@ -977,7 +987,7 @@ __global__ void k_resolve(PassArgs a, TableOf<MS> tab) {
             if (o.accum) {
                 o.accum[3 * (size_t)px] += lp.x; o.accum[3 * (size_t)px + 1] += lp.y; o.accum[3 * (size_t)px + 2] += lp.z;
             }
-            const uint32_t flags = a.ws.st[p].y;
+            const uint32_t flags = nrc || o.thr_out ? a.ws.st[p].y : 0u;
             const bool rec = nrc && (flags & F_TRAIN) && (flags & F_CAPTURED);
             const bool head_query = rec && !(flags & F_FULL);
             if (o.thr_out && !(flags & F_INF) && !head_query) o.thr_out[px] = TfgColor{0.0f, 0.0f, 0.0f};
@@ -1129,8 +1139,8 @@ int shapes_for(int dev, LaunchShapes& s) {
             g.shadow_occ[1][0][k] = occ_of(k_shadow<0, false, true>, bt, sm_ms);
             g.shadow_occ[1][1][k] = occ_of(k_shadow<1, false, true>, bt, sm_ms);
         }
-        g.shade_blocks[0] = sms * occ_of(k_shade<false>, 256, 0);
-        g.shade_blocks[1] = sms * occ_of(k_shade<true>, 256, 0);
+        g.shade_blocks[0] = sms * occ_of(k_shade<false>, kShadeThreads, 0);
+        g.shade_blocks[1] = sms * occ_of(k_shade<true>, kShadeThreads, 0);
         g.few_occ[0][0] = occ_of(k_few<0, false>, kFewThreads, 0);
         g.few_occ[0][1] = occ_of(k_few<1, false>, kFewThreads, 0);
         g.few_occ[1][0] = occ_of(k_few<0, true>, kFewThreads, 0);
@@ -1552,7 +1562,8 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
         if (few_ok && a.nq <= kFewPaths) {
             for (int b = 0; b < prm.max_depth; ++b) {
                 few(b, b - 1, 1, (b == 0 ? 1u : 1u + few_points) * a.nq, stream);
-                launch(k_shade<MS>, std::min((uint32_t)shade_grid, (a.nq + 255u) / 256u), 256u, stream, true, a, b, tab);
+                launch(k_shade<MS>, std::min((uint32_t)shade_grid, (a.nq + kShadeThreads - 1u) / kShadeThreads),
+                       (uint32_t)kShadeThreads, stream, true, a, b, tab);
             }
             few(-1, prm.max_depth - 1, 1, few_points * a.nq, stream);
             launch(k_resolve<MS>, (uint32_t)res_blocks, 256u, stream, true, a, tab);
@@ -1576,7 +1587,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
                 e = cudaStreamWaitEvent(stream, ws.join[b - 1], 0);
                 if (e != cudaSuccess) return fail((int)e, cudaGetErrorString(e));
             }
-            stage(2, [&] { k_shade<MS><<<shade_grid, 256, 0, stream>>>(a, b, tab); });
+            stage(2, [&] { k_shade<MS><<<shade_grid, kShadeThreads, 0, stream>>>(a, b, tab); });
             if (overlap) {
                 e = cudaEventRecord(ws.fork[b], stream);
                 if (e == cudaSuccess) e = cudaStreamWaitEvent(sstream, ws.fork[b], 0);
