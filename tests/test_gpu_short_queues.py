@@ -140,12 +140,13 @@ def test_batches_with_short_queues(built, sizes):
         d.close()
 
 
-def test_passes_that_follow_each_other_closely(built):
+@pytest.mark.parametrize("w,h", [(64, 48), (300, 256)])   # k_few alone; beside the long-queue kernels
+def test_passes_that_follow_each_other_closely(built, w, h):
     """Kernels of short wavefronts start before their predecessors end: passes
     back to back, in several wavefronts each, with writes to what they read
     between them, directly and as a replayed graph."""
-    ds = pt.DeviceScene(scenes.reference_room(64, 48, subdiv=2), "cuda")
-    n = 64 * 48
+    ds = pt.DeviceScene(scenes.reference_room(w, h, subdiv=2), "cuda")
+    n = w * h
     p = pt.RenderParams(max_depth=6, rr_min_depth=3, shadow_mesh=1, spp=2, accumulate=1)
     imgs = [torch.zeros(n * 3, device="cuda") for _ in range(4)]
     acc = torch.zeros(n * 3, device="cuda")
@@ -166,7 +167,7 @@ def test_passes_that_follow_each_other_closely(built):
         torch.cuda.synchronize()
     want = [acc.clone()] + [i.clone() for i in imgs]
 
-    for wavefront in (0, 1024):
+    for wavefront in (0, n // 3):
         pt.set_tuning(pt.RenderTuning.default() if not wavefront else pt.RenderTuning(wavefront_paths=wavefront))
         passes()
         torch.cuda.synchronize()

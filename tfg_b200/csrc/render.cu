@@ -155,13 +155,15 @@ struct Outs {
 // nothing from it, and waits for it here; then it lets its own successor
 // start, so that by the time any kernel runs, all but its predecessor have
 // finished.  Both calls do nothing in kernels launched the ordinary way.
-// A 128 x 128 sample is 22 such kernels of 5 to 20 us each: 430 us with
+// A 128 x 128 sample of 20 bounces is 43 kernels of 4 to 19 us: 430 us with
 // ordinary launches, 350 us so.  k_generate does not let its successor in
 // early: 357 us.
 __device__ __forceinline__ void pdl_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
@@ -390,6 +392,7 @@ __global__ void k_generate(PassArgs a, TableOf<MS> tab) {
 template <int TRI_FMT, bool STATS, bool MS>
 __global__ void __launch_bounds__(256, MS && !STATS ? 4 : 0) k_trace(PassArgs a, int bounce, TableOf<MS> tab) {
     extern __shared__ unsigned char smem_raw[];
+    if (a.few_max) pdl_launch();   // k_few, beside
     uint2* sstack = reinterpret_cast<uint2*>(smem_raw);
     APrim* sprims = reinterpret_cast<APrim*>(smem_raw + sizeof(uint2) * kSmemStack * blockDim.x);
     // one scene: its analytic primitives are cached in shared memory
@@ -508,7 +511,7 @@ __device__ __forceinline__ void write_datos(TfgDatosMLP* d, V3 P, V3 dir, V3 n, 
 // its primitive are requested together (load_prim), and radiance is read and
 // written only where it changes.  Blocks of 128 spread short queues over more
 // SMs and fill the register file better than 256.  With the same in k_resolve
-// (flags read only for the cache): 128 x 128 350 -> 330 us, 16 samples of
+// (flags read only for the cache): 128 x 128 350 -> 330 us, 4 samples of
 // 1920 x 1080 10.55 -> 10.38 ms.  More warps by a register limit: 6 blocks per
 // SM 10.9 ms, 7 10.9, 8 11.0.
 constexpr int kShadeThreads = 128;
@@ -777,6 +780,7 @@ __device__ __forceinline__ uint32_t few_rays_per_point(int nl) {
 
 template <int TRI_FMT, bool STATS, bool MS>
 __global__ void __launch_bounds__(256, (MS || TRI_FMT == 0) && !STATS ? 4 : 0) k_shadow(PassArgs a, int bounce, TableOf<MS> tab) {
+    if (a.few_max) pdl_launch();   // k_few, beside
     extern __shared__ unsigned char smem_raw[];
     uint2* sstack = reinterpret_cast<uint2*>(smem_raw);
     APrim* sprims = reinterpret_cast<APrim*>(smem_raw + sizeof(uint2) * kSmemStack * blockDim.x);
@@ -863,7 +867,8 @@ __global__ void __launch_bounds__(256, (MS || TRI_FMT == 0) && !STATS ? 4 : 0) k
 // All groups take rays first to last and shading points last to first, so
 // that with room for both they run side by side.  `always`: whatever the
 // queues' lengths (a wavefront that starts short); else only what k_trace /
-// k_shadow leave (a.few_max).
+// k_shadow leave (a.few_max); then it starts beside the kernel it completes, whose
+// queue is the same and of which only one does the work, and ends after it.
 constexpr int kFewThreads = 128;
 
 template <int TRI_FMT, bool MS>
@@ -871,8 +876,11 @@ __global__ void __launch_bounds__(kFewThreads, 8) k_few(PassArgs a, int tb, int 
     __shared__ uint2 sstack[kStackTotal * kFewThreads / 8];
     __shared__ APrim sprims[MS ? 1 : kSmemPrims];
     const uint32_t P = few_rays_per_point<MS>(a.nlights);
-    const int nsm = MS ? 0 : load_aprims_smem(sprims, a.prims, a.nprims);   // no kernel of the wavefront writes these
-    pdl_sync();
+    int nsm = 0;
+    if (always) {
+        if (!MS) nsm = load_aprims_smem(sprims, a.prims, a.nprims);   // no kernel of the wavefront writes these
+        pdl_sync();
+    }
     uint32_t n_rays = 0, n_points = 0;
     if (tb >= 0) {
         n_rays = a.ws.counters[4 * tb + 0];
@@ -882,7 +890,11 @@ __global__ void __launch_bounds__(kFewThreads, 8) k_few(PassArgs a, int tb, int 
         n_points = a.ws.counters[4 * sb + 2];
         if (!always && n_points * P > a.few_max) n_points = 0;
     }
-    if (n_rays == 0 && n_points == 0) return;
+    if (n_rays == 0 && n_points == 0) {
+        pdl_wait();
+        return;
+    }
+    if (!MS && !always) nsm = load_aprims_smem(sprims, a.prims, a.nprims);
     Geo g = geo_of<MS>(a, tab, 0);
     uint2* stack = sstack + threadIdx.x / 8u;
     constexpr int kStride = kFewThreads / 8;
@@ -952,6 +964,7 @@ __global__ void __launch_bounds__(kFewThreads, 8) k_few(PassArgs a, int tb, int 
             }
         }
     }
+    pdl_wait();
 }
 
 // ------------------------------------------------------------------ resolve
@@ -1516,7 +1529,10 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     // k_few for short queues: alone, closest hits and the previous bounce's
     // shadow rays in one launch, for wavefronts that start short; beside the
     // long-queue kernels from bounce kFewFrom on otherwise (the queue lengths
-    // are only known on the device; a launch with nothing to do takes ~2 us).
+    // are only known on the device).  There it starts beside the kernel whose
+    // short queues it takes and waits for that one's end only at its own:
+    // launched after it, the empty launches of a 20-bounce 906 x 562 sample cost
+    // 42 us of 1,356.
     // Stage timing and work counts keep the stages apart.
     const uint32_t few_groups = (uint32_t)(sh.sms * sh.few_occ[MS][fmt]) * (kFewThreads / 8u);
     const bool few_ok = !times && !counts;
@@ -1537,8 +1553,8 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     auto few = [&](int tb, int sb, int always, uint32_t tasks, cudaStream_t st) {
         const uint32_t fit = (uint32_t)(sh.sms * sh.few_occ[MS][fmt]);
         const uint32_t grid = std::max(1u, std::min(fit, (tasks + kFewThreads / 8u - 1) / (kFewThreads / 8u)));
-        if (fmt == 0) launch(k_few<0, MS>, grid, kFewThreads, st, always != 0, a, tb, sb, always, tab);
-        else launch(k_few<1, MS>, grid, kFewThreads, st, always != 0, a, tb, sb, always, tab);
+        if (fmt == 0) launch(k_few<0, MS>, grid, kFewThreads, st, true, a, tb, sb, always, tab);
+        else launch(k_few<1, MS>, grid, kFewThreads, st, true, a, tb, sb, always, tab);
     };
     a.frame = frame;
     a.img = img;
