@@ -891,7 +891,7 @@ __global__ void __launch_bounds__(kFewThreads, 8) k_few(PassArgs a, int tb, int 
         if (!always && n_points * P > a.few_max) n_points = 0;
     }
     if (n_rays == 0 && n_points == 0) {
-        pdl_wait();
+        if (blockIdx.x == 0) pdl_wait();   // one block holds the launch's end; the others leave their SM to the rest
         return;
     }
     if (!MS && !always) nsm = load_aprims_smem(sprims, a.prims, a.nprims);
@@ -1532,7 +1532,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     // are only known on the device).  There it starts beside the kernel whose
     // short queues it takes and waits for that one's end only at its own:
     // launched after it, the empty launches of a 20-bounce 906 x 562 sample cost
-    // 42 us of 1,356.
+    // 52 us of 1,356.
     // Stage timing and work counts keep the stages apart.
     const uint32_t few_groups = (uint32_t)(sh.sms * sh.few_occ[MS][fmt]) * (kFewThreads / 8u);
     const bool few_ok = !times && !counts;
