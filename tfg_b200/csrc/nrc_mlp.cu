@@ -505,12 +505,12 @@ __device__ __forceinline__ float scrub(float c) {
 
 // A step's kernels are launched with programmatic stream serialisation: a
 // kernel lets the next one start (pdl_launch), and the next one sets itself up
-// and waits for the kernel before it to have finished, its writes visible
-// (pdl_wait).  Two rules keep the chain in order.  A kernel's end implies its
-// predecessors': every block waits before it ends.  And a kernel that touches
-// global memory before its wait, or waits only at its end, starts behind one
-// that calls pdl_launch after its own wait, so that all earlier kernels have
-// finished.  Both calls do nothing in kernels launched the ordinary way.
+// (barriers, TMEM, zeroed stages) and waits for the kernel before it to have
+// finished, its writes visible (pdl_wait).  Every block waits before it touches
+// global memory, also memory that only earlier kernels of the stream wrote --
+// their writes are promised to be visible to a kernel that has waited, not to
+// one that started early -- and before it ends, so that a kernel's end implies
+// its predecessors'.  Both calls do nothing in kernels launched the ordinary way.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -1872,9 +1872,6 @@ struct WgradArgs {
     uint32_t loss_ctas;
     float* loss;
     float inv_count;
-    // The kernel before is the table gradient, which this one runs beside; it
-    // waits for it at its end.
-    int beside;
 };
 
 // Ends a step: advance the step counter and Adam time, keep a running loss.
@@ -1912,11 +1909,10 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = tslot;
-    if (!a.beside) pdl_wait();
-    pdl_launch();   // after the wait: k_adam reads the masters before its own
+    pdl_wait();
+    pdl_launch();
     const uint32_t navail = a.state[S_NAVAIL];
     if (navail < a.min_n || navail == 0) {
-        pdl_wait();
         if (warp == 0) umma::tmem_dealloc(tmem, 128);
         return;
     }
@@ -1989,7 +1985,6 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
         }
     }
     if (!ok && t == 0) atomicExch(&g_mlp_error, 1);
-    if (a.beside) pdl_wait();
     if (warp == 3 && blockIdx.x == 0 && blockIdx.y == 0) {
         float sum = 0.0f;
         for (uint32_t k = (uint32_t)(t & 31); k < a.loss_ctas; k += 32u) sum += a.loss_part[k];
@@ -2055,18 +2050,16 @@ __device__ __forceinline__ void layer_of(int i, int& l, int& r, int& c) {
 template <int NL, int HID>
 __global__ void k_adam(AdamArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= params_h<HID>(NL)) { pdl_wait(); return; }
+    pdl_wait();
+    pdl_launch();
+    if (i >= params_h<HID>(NL)) return;
     int l, r, c;
     layer_of<NL, HID>(i, l, r, c);
     // Padded entries (output rows 3..15, input columns past the encoding of layer 0) stay zero.
     const bool live = !(l == NL - 1 && r >= 3) && !(l == 0 && c >= a.live0);
-    // masters, moments and average are this kernel's own: read them while the
-    // gradients are still being formed
     float w = a.w[i];
     float e = a.ema[i];
     const float m0 = a.m[i], v0 = a.v[i];
-    pdl_wait();
-    pdl_launch();   // after the wait: the tables' Adam kernel waits for this one only at its end
     const bool update = a.update && a.state[S_NAVAIL] >= a.min_n && a.state[S_NAVAIL] > 0;
     const float tn = (float)(a.state[S_ADAM_T] + ((update && !a.ticked) ? 1u : 0u));
     if (update && live) {
@@ -2132,7 +2125,7 @@ __global__ void __launch_bounds__(kHashGradThreads) k_hash_grad(HashGradArgs a) 
     __shared__ float sw[128][2 * kHashMaxLevels];
     __shared__ float sdz[kHashGradSamples][128 + 1];
     pdl_wait();
-    pdl_launch();   // after the wait: k_wgrad waits for this kernel only at its end
+    pdl_launch();
     const int L2 = 2 * a.hg.levels;
     for (int i = threadIdx.x; i < a.hid * 2 * kHashMaxLevels; i += blockDim.x) {
         const int o = i / (2 * kHashMaxLevels), j = i % (2 * kHashMaxLevels);
@@ -2236,7 +2229,7 @@ __device__ __forceinline__ bool bits_differ(const float4& a, const float4& b) {
 // -- a step's samples touch about a tenth of the entries, the gradient of the
 // others is zero already, and entries no sample ever touched keep all three.
 __global__ void __launch_bounds__(256, 4) k_adam_hash(HashAdamArgs a) {
-    // (runs beside the layers' Adam kernel, which has waited for both gradients)
+    pdl_wait();
     const bool update = a.update && a.state[S_NAVAIL] >= a.min_n && a.state[S_NAVAIL] > 0;
     const float tn = (float)a.state[S_ADAM_T];   // k_wgrad has ended the step
     HashAdamStep st{a.lr, a.beta1, a.beta2, a.eps, a.decay, a.grad_scale,
@@ -2281,7 +2274,6 @@ __global__ void __launch_bounds__(256, 4) k_adam_hash(HashAdamArgs a) {
         a.infer[i] = __float2half_rn(r);
     }
     pdl_launch();
-    pdl_wait();
 }
 
 // Initial table values: uniform in (-1e-4, 1e-4) (Mueller et al. 2022),
@@ -2595,10 +2587,9 @@ uint32_t infer_grid(const ColorMlp* n, uint32_t tiles) {
 }
 
 // Weight gradients of the batch the last forward / backward kernel ran.
-// `in_step`: launched early behind the step's previous kernel (the forward /
-// backward kernel, or with `beside` the table gradient that it runs beside).
+// `in_step`: launched early behind the step's previous kernel.
 int enqueue_wgrad(ColorMlp* n, uint32_t tiles_per_cta, uint32_t min_n, cudaStream_t s, bool in_step = false,
-                  bool beside = false, bool tick = false) {
+                  bool tick = false) {
     const uint32_t tiles = n->batch / mlp::kTile;
     mlp::WgradArgs wa;
     for (int l = 0; l < mlp::kMaxLayers; ++l) { wa.zT[l] = n->zT[l]; wa.hT[l] = n->hT[l]; }
@@ -2609,7 +2600,6 @@ int enqueue_wgrad(ColorMlp* n, uint32_t tiles_per_cta, uint32_t min_n, cudaStrea
     wa.loss_part = n->loss + 1;
     wa.loss_ctas = std::min<uint32_t>(tiles, (uint32_t)n->sms);
     wa.loss = n->loss;
-    wa.beside = beside ? 1 : 0;
     wa.inv_count = 1.0f / (3.0f * (float)n->batch);
     const uint32_t groups = (tiles + wa.tiles_per_cta - 1) / wa.tiles_per_cta;
     cudaError_t e = cudaSuccess;
@@ -2662,9 +2652,8 @@ int enqueue_step(ColorMlp* n, const TfgDatosMLP* buf, uint32_t min_n, bool updat
     });
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "mlp step: forward/backward");
-    // The table gradient (atomics), which re-draws the step's samples from its
-    // seed, runs beside the weight gradients (tensor cores, 96 CTAs), whose
-    // kernel ends the step; then the two Adam kernels run side by side.
+    // The table gradient re-draws the step's samples from its seed, so it comes
+    // before the weight gradients, whose kernel ends the step.
     if (n->hlevels) {
         mlp::HashGradArgs ha;
         ha.buf = buf; ha.state = n->dstate; ha.min_n = min_n; ha.batch = n->batch; ha.bounds = n->bounds;
@@ -2674,7 +2663,7 @@ int enqueue_step(ColorMlp* n, const TfgDatosMLP* buf, uint32_t min_n, bool updat
                          mlp::kHashGradThreads, 0, s, ha);
         if (e != cudaSuccess) return cuda_fail(e, "mlp step: table gradient");
     }
-    if (int rc = enqueue_wgrad(n, wgrad_tiles_per_cta(n, tiles), min_n, s, true, n->hlevels != 0, update)) return rc;
+    if (int rc = enqueue_wgrad(n, wgrad_tiles_per_cta(n, tiles), min_n, s, true, update)) return rc;
     if (!update) return enqueue_wgrad_sum(n, min_n, s);
     if (int rc = enqueue_adam(n, s, true, min_n)) return rc;
     return enqueue_adam_hash(n, s, true, min_n);
