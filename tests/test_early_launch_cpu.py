@@ -35,7 +35,7 @@ def _touched_before_wait(body: str, wait: str) -> list[str]:
     return seen + ["no unconditional %s()" % wait]
 
 
-@pytest.mark.parametrize("kernel", ["k_train", "k_train128", "k_hash_grad", "k_wgrad", "k_adam", "k_adam_hash"])
+@pytest.mark.parametrize("kernel", ["k_train", "k_train128", "k_wgrad", "k_adam", "k_adam_hash"])
 def test_training_kernels_wait_first(kernel):
     src = (CSRC / "nrc_mlp.cu").read_text()
     assert "launch_early(mlp::%s" % kernel in src
@@ -45,4 +45,4 @@ def test_training_kernels_wait_first(kernel):
 def test_no_other_training_kernel_is_launched_early():
     src = (CSRC / "nrc_mlp.cu").read_text()
     names = set(re.findall(r"launch_early\(mlp::(\w+)", src))
-    assert names == {"k_train", "k_train128", "k_hash_grad", "k_wgrad", "k_adam", "k_adam_hash"}
+    assert names == {"k_train", "k_train128", "k_wgrad", "k_adam", "k_adam_hash"}

@@ -250,46 +250,34 @@ __device__ __forceinline__ void level_rows(const uint32_t (&i)[3], uint32_t n_ce
     }
 }
 
-// The hash-grid features of levels L0 .. L0 + N - 1 at position p from the
-// FP32 tables (the training forward pass), two per level; all 8 N corner
-// loads are issued before a level is combined.  A level's trilinear sum runs
-// over its four (y, z) corner rows: each row's x pair is blended with the x
-// weights, then the row with its (y, z) weight.
-template <int L0, int N>
-__device__ __forceinline__ void hash_features(const float (&p)[3], const HashGrid& g, float* h) {
+// The 2L hash-grid features of position p from the FP32 tables (the training
+// forward pass).  A level's trilinear sum runs over its four (y, z) corner
+// rows: each row's x pair is blended with the x weights, then the row with
+// its (y, z) weight.
+__device__ __forceinline__ void hash_features(const float (&p)[3], const HashGrid& g, float (&h)[2 * kHashMaxLevels]) {
 #pragma unroll
-    for (int k = 0; k < 2 * N; ++k) h[k] = 0.0f;
-    if (L0 >= g.levels) return;
-    float2 v[N][8];
-    float f[N][3];
-#pragma unroll
-    for (int b = 0; b < N; ++b) {
-        // a level past the last (resolution 0, hashed) reads the last one's
-        // table and is dropped below
-        const int l = L0 + b;
+    for (int l = 0; l < kHashMaxLevels; ++l) {
+        h[2 * l] = 0.0f;
+        h[2 * l + 1] = 0.0f;
+        if (l >= g.levels) continue;
         const float n = g.res[l];
         uint32_t i[3], o0[4], o1[4];
-        hash_cell(p, n, i, f[b]);
+        float f[3];
+        hash_cell(p, n, i, f);
         level_rows<8>(i, (uint32_t)n, (g.dense >> l) & 1u, g.T, o0, o1);
-        const char* lvl = reinterpret_cast<const char*>(g.master + (size_t)min(l, g.levels - 1) * g.T);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            v[b][2 * r] = __ldg(reinterpret_cast<const float2*>(lvl + o0[r]));
-            v[b][2 * r + 1] = __ldg(reinterpret_cast<const float2*>(lvl + o1[r]));
-        }
-    }
-#pragma unroll
-    for (int b = 0; b < N; ++b) {
-        const float wx0 = 1.0f - f[b][0], wy0 = 1.0f - f[b][1], wz0 = 1.0f - f[b][2];
+        const char* lvl = reinterpret_cast<const char*>(g.master + (size_t)l * g.T);
+        const float wx0 = 1.0f - f[0], wy0 = 1.0f - f[1], wz0 = 1.0f - f[2];
         float a0 = 0.0f, a1 = 0.0f;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const float2 v0 = v[b][2 * r], v1 = v[b][2 * r + 1];
-            const float wyz = ((r & 1) ? f[b][1] : wy0) * ((r & 2) ? f[b][2] : wz0);
-            a0 = fmaf(wyz, fmaf(f[b][0], v1.x, wx0 * v0.x), a0);
-            a1 = fmaf(wyz, fmaf(f[b][0], v1.y, wx0 * v0.y), a1);
+            const float2 v0 = __ldg(reinterpret_cast<const float2*>(lvl + o0[r]));
+            const float2 v1 = __ldg(reinterpret_cast<const float2*>(lvl + o1[r]));
+            const float wyz = ((r & 1) ? f[1] : wy0) * ((r & 2) ? f[2] : wz0);
+            a0 = fmaf(wyz, fmaf(f[0], v1.x, wx0 * v0.x), a0);
+            a1 = fmaf(wyz, fmaf(f[0], v1.y, wx0 * v0.y), a1);
         }
-        if (L0 + b < g.levels) { h[2 * b] = a0; h[2 * b + 1] = a1; }
+        h[2 * l] = a0;
+        h[2 * l + 1] = a1;
     }
 }
 
@@ -398,10 +386,7 @@ __device__ __forceinline__ void composite_features(const TfgDatosMLP& d, const B
     float p[3];
     unit_position(d, b, p);
     float h[2 * kHashMaxLevels], t[32];
-    hash_features<0, 4>(p, g, h);
-    hash_features<4, 4>(p, g, h + 8);
-    hash_features<8, 4>(p, g, h + 16);
-    hash_features<12, 4>(p, g, h + 24);
+    hash_features(p, g, h);
     composite_tail(d, t);
 #pragma unroll
     for (int k = 0; k < 32; ++k) {
@@ -2124,7 +2109,6 @@ constexpr int kHashGradSamples = kHashGradThreads / kHashMaxLevels;
 __global__ void __launch_bounds__(kHashGradThreads) k_hash_grad(HashGradArgs a) {
     __shared__ float sw[128][2 * kHashMaxLevels];
     __shared__ float sdz[kHashGradSamples][128 + 1];
-    pdl_wait();
     pdl_launch();
     const int L2 = 2 * a.hg.levels;
     for (int i = threadIdx.x; i < a.hid * 2 * kHashMaxLevels; i += blockDim.x) {
@@ -2199,36 +2183,23 @@ struct HashAdamArgs {
 struct HashAdamStep {
     float lr, beta1, beta2, eps, decay, grad_scale, inv_bc1, inv_bc2, inv_debias;
     bool update;
-    // Sums are fused as written, whatever surrounds them.  (PLAIN: the
-    // gradient's product is rounded and the moment's fused, as the compiler
-    // had it for the first of four values before this was written out; kept, so
-    // that training gives the same tables to the bit.)
-    template <bool PLAIN>
-    __device__ __forceinline__ float run(float& w, float& m, float& v, float& e, float g) const {
+    __device__ __forceinline__ float operator()(float& w, float& m, float& v, float& e, float g) const {
         if (update) {
             g *= grad_scale;
-            m = PLAIN ? __fmaf_rn(beta1, m, __fmul_rn(1.0f - beta1, g)) : __fmaf_rn(1.0f - beta1, g, __fmul_rn(beta1, m));
-            v = __fmaf_rn(__fmul_rn(1.0f - beta2, g), g, __fmul_rn(beta2, v));
+            m = beta1 * m + (1.0f - beta1) * g;
+            v = beta2 * v + (1.0f - beta2) * g * g;
             w -= lr * (m * inv_bc1) / (sqrtf(v * inv_bc2) + eps);
-            e = __fmaf_rn(decay, e, __fmul_rn(1.0f - decay, w));
+            e = decay * e + (1.0f - decay) * w;
         }
         return inv_debias > 0.0f ? e * inv_debias : w;
     }
 };
 
-__device__ __forceinline__ bool bits_differ(const float4& a, const float4& b) {
-    return ((__float_as_uint(a.x) ^ __float_as_uint(b.x)) | (__float_as_uint(a.y) ^ __float_as_uint(b.y)) |
-            (__float_as_uint(a.z) ^ __float_as_uint(b.z)) | (__float_as_uint(a.w) ^ __float_as_uint(b.w))) != 0u;
-}
-
 // Four values per thread and iteration (16-byte loads and stores of every
 // array; the arrays are separate allocations, so 16-byte aligned), then a
-// scalar tail.  HBM-bound: gradient, moments, masters and average are read
-// once (20 bytes per value) and the average and its FP16 image written once;
-// gradient, moments and masters are written only where a bit of them changed
-// -- a step's samples touch about a tenth of the entries, the gradient of the
-// others is zero already, and entries no sample ever touched keep all three.
-__global__ void __launch_bounds__(256, 4) k_adam_hash(HashAdamArgs a) {
+// scalar tail.  Gradient, moments, masters and average are read once and
+// written once: 38 bytes per value.
+__global__ void k_adam_hash(HashAdamArgs a) {
     pdl_wait();
     const bool update = a.update && a.state[S_NAVAIL] >= a.min_n && a.state[S_NAVAIL] > 0;
     const float tn = (float)a.state[S_ADAM_T];   // k_wgrad has ended the step
@@ -2243,36 +2214,27 @@ __global__ void __launch_bounds__(256, 4) k_adam_hash(HashAdamArgs a) {
     float4* e4 = reinterpret_cast<float4*>(a.ema);
     float4* g4 = reinterpret_cast<float4*>(a.grad);
     uint2* i4 = reinterpret_cast<uint2*>(a.infer);
-    // odd steps run the arrays backwards: the end of the step before is still
-    // in L2
-    const bool back = a.state[S_ADAM_T] & 1u;
-    for (size_t k = t0; k < n4; k += stride) {
-        const size_t i = back ? n4 - 1 - k : k;
+    for (size_t i = t0; i < n4; i += stride) {
         float4 w = w4[i], e = e4[i];
         const float4 g = g4[i];
         float4 m = make_float4(0.f, 0.f, 0.f, 0.f), v = m;
         if (update) { m = m4[i]; v = v4[i]; }
-        const float4 w0 = w, m0 = m, v0 = v;
-        const float r0 = st.run<true>(w.x, m.x, v.x, e.x, g.x), r1 = st.run<false>(w.y, m.y, v.y, e.y, g.y);
-        const float r2 = st.run<false>(w.z, m.z, v.z, e.z, g.z), r3 = st.run<false>(w.w, m.w, v.w, e.w, g.w);
-        if (update) {
-            if (bits_differ(m, m0)) m4[i] = m;
-            if (bits_differ(v, v0)) v4[i] = v;
-            if (bits_differ(w, w0)) w4[i] = w;
-            e4[i] = e;
-        }
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (bits_differ(g, zero)) g4[i] = zero;
+        const float r0 = st(w.x, m.x, v.x, e.x, g.x), r1 = st(w.y, m.y, v.y, e.y, g.y);
+        const float r2 = st(w.z, m.z, v.z, e.z, g.z), r3 = st(w.w, m.w, v.w, e.w, g.w);
+        if (update) { m4[i] = m; v4[i] = v; w4[i] = w; e4[i] = e; }
+        g4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         __half2 h01 = __floats2half2_rn(r0, r1), h23 = __floats2half2_rn(r2, r3);
         i4[i] = make_uint2(*reinterpret_cast<uint32_t*>(&h01), *reinterpret_cast<uint32_t*>(&h23));
     }
     for (size_t i = 4 * n4 + t0; i < a.count; i += stride) {
         float w = a.w[i], m = update ? a.m[i] : 0.0f, v = update ? a.v[i] : 0.0f, e = a.ema[i];
-        const float r = st.run<false>(w, m, v, e, a.grad[i]);
+        const float r = st(w, m, v, e, a.grad[i]);
         if (update) { a.m[i] = m; a.v[i] = v; a.w[i] = w; a.ema[i] = e; }
         a.grad[i] = 0.0f;
         a.infer[i] = __float2half_rn(r);
     }
+    // (only here: after the wait, the next step's CTAs would take the room of the
+    // blocks still to come -- four steps 915 us, 888 so)
     pdl_launch();
 }
 
@@ -2520,9 +2482,7 @@ int enqueue_adam_hash(ColorMlp* n, cudaStream_t s, bool update, uint32_t min_n) 
     h.lr = n->lr; h.beta1 = n->beta1; h.beta2 = n->beta2; h.eps = n->eps; h.decay = n->decay;
     h.grad_scale = 1.0f / (3.0f * (float)n->batch);
     h.state = n->dstate; h.min_n = min_n; h.update = update ? 1 : 0;
-    // four blocks fit an SM; eight rounds of them (four training steps of the
-    // reference's tables: 862 us; 871 with four rounds, 888 with one)
-    const unsigned blocks = (unsigned)std::min<size_t>((n->hcount + 255) / 256, (size_t)n->sms * 32);
+    const unsigned blocks = (unsigned)std::min<size_t>((n->hcount + 255) / 256, (size_t)n->sms * 16);
     cudaError_t e = cudaSuccess;
     if (update) e = launch_early(mlp::k_adam_hash, dim3(blocks), 256, 0, s, h);
     else mlp::k_adam_hash<<<blocks, 256, 0, s>>>(h);
@@ -2659,8 +2619,11 @@ int enqueue_step(ColorMlp* n, const TfgDatosMLP* buf, uint32_t min_n, bool updat
         ha.buf = buf; ha.state = n->dstate; ha.min_n = min_n; ha.batch = n->batch; ha.bounds = n->bounds;
         ha.zT0 = n->zT[0]; ha.w0 = n->w; ha.grad = reinterpret_cast<float2*>(n->hgrad); ha.hg = hash_view(n, true);
         ha.hid = n->hid;
-        e = launch_early(mlp::k_hash_grad, dim3((n->batch + mlp::kHashGradSamples - 1) / mlp::kHashGradSamples),
-                         mlp::kHashGradThreads, 0, s, ha);
+        // (launched the ordinary way: started early, all blocks wait and then
+        // begin together, and the atomics' order varies twice as much from run to
+        // run; four steps 895 us so, 900 like this)
+        mlp::k_hash_grad<<<(n->batch + mlp::kHashGradSamples - 1) / mlp::kHashGradSamples, mlp::kHashGradThreads, 0, s>>>(ha);
+        e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "mlp step: table gradient");
     }
     if (int rc = enqueue_wgrad(n, wgrad_tiles_per_cta(n, tiles), min_n, s, true, update)) return rc;
