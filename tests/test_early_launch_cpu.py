@@ -46,3 +46,31 @@ def test_no_other_training_kernel_is_launched_early():
     src = (CSRC / "nrc_mlp.cu").read_text()
     names = set(re.findall(r"launch_early\(mlp::(\w+)", src))
     assert names == {"k_train", "k_train128", "k_wgrad", "k_adam", "k_adam_hash"}
+
+
+@pytest.mark.parametrize("kernel", ["k_shade", "k_resolve"])
+def test_render_kernels_wait_first(kernel):
+    assert _touched_before_wait(_body((CSRC / "render.cu").read_text(), kernel), "pdl_sync") == []
+
+
+def test_short_queue_kernel_waits_or_acquires_first():
+    src = (CSRC / "render.cu").read_text()
+    body = _body(src, "k_few")
+    head, rest = body.split("    if (always) {\n", 1)
+    assert TOUCH.findall(head) == [] and rest.lstrip().startswith("pdl_sync();")
+    beside = rest.split("    } else {", 1)[1].split("    }\n", 1)[0]
+    assert "handed_over(" in beside.split(";")[0]
+    # the length comes with acquire semantics, or after a wait; it was released before k_few could start
+    take = src[src.index("uint32_t handed_over("):]
+    take = take[:take.index("\n}\n")]
+    assert take.index("ld.acquire.gpu") < take.index("pdl_wait();") < take.index("return counters[")
+    give = src[src.index("void hand_over("):]
+    give = give[:give.index("\n}\n")]
+    assert give.index("st.release.gpu") < give.index("__syncthreads();") < give.index("pdl_launch();")
+    for kernel in ("k_trace", "k_shadow"):
+        assert "pdl_launch" not in _body(src, kernel) and "hand_over(" in _body(src, kernel)
+
+
+def test_no_other_render_kernel_is_launched_early():
+    src = (CSRC / "render.cu").read_text()
+    assert set(re.findall(r"[ (]launch\((\w+)<", src)) == {"k_few", "k_shade", "k_resolve"}
