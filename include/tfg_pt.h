@@ -332,7 +332,8 @@ typedef struct TfgRenderTuning {
     int32_t wavefront_paths;    /* queue capacity: paths per wavefront.  0 (default) = the call's samples
                                    spread evenly over wavefronts of at most 2^24 paths and an eighth of
                                    the free device memory, at least one sample of every pixel (W*H) --
-                                   exactly one under stream capture.  More runs several samples of the
+                                   exactly one under stream capture, for which an uncaptured call with
+                                   the same image size has made room.  More runs several samples of the
                                    call per launch, less splits a sample into chunks; passes that query
                                    or train the cache stop at W*H.  0 or 1024 .. 2^26 (224 B of device
                                    memory per path) */

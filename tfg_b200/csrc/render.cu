@@ -1253,7 +1253,9 @@ Tuning resolve_tuning(int dev, uint32_t npix, int spp, bool nrc, uint32_t* gener
 // of the device's free memory (fewer samples per wavefront beyond that).  One
 // sample at a time on the caller's slot is the fall-back -- under stream
 // capture, where nothing may be allocated and the captured pass must keep its
-// queues as long as it always did, and when the allocation fails.
+// queues as long as it always did, and when the allocation fails.  So a widened
+// call sizes the caller's slot, too: the call that warms a pass up is the call
+// that is captured next.
 int pass_workspace(int dev, int slot, uint32_t npix, int spp, bool nrc, cudaStream_t stream, Tuning& tu,
                    Workspace& ws) {
     if (tu.widened) {
@@ -1261,6 +1263,8 @@ int pass_workspace(int dev, int slot, uint32_t npix, int spp, bool nrc, cudaStre
         const cudaError_t e = cudaStreamIsCapturing(stream, &cap);
         bool wide = e == cudaSuccess && cap == cudaStreamCaptureStatusNone;
         if (e != cudaSuccess) cudaGetLastError();
+        if (wide)
+            if (int rc = ensure_workspace(dev, slot, npix, nrc, ws)) return rc;
         size_t have = 0;
         {
             std::lock_guard<std::mutex> lk(g_ws_mutex);
