@@ -1084,6 +1084,11 @@ namespace {
 // captured pass) that runs one sample at a time.
 constexpr int kWideSlot = kWorkspaceSlots;
 std::mutex g_ws_mutex;
+// Held by a pass from the moment it knows its queues until its last launch is
+// enqueued: a call on another host thread that needs larger queues frees these,
+// which waits for launched work, not for work about to be launched.  A call that
+// takes two slots locks the wide one last.
+std::mutex g_pass_mutex[kMaxDevices][kWorkspaceSlots + 1];
 Workspace g_ws[kMaxDevices][kWorkspaceSlots + 1];
 
 int ensure_workspace(int dev, int slot, size_t paths, bool nrc, Workspace& out) {
@@ -1256,8 +1261,16 @@ Tuning resolve_tuning(int dev, uint32_t npix, int spp, bool nrc, uint32_t* gener
 // queues as long as it always did, and when the allocation fails.  So a widened
 // call sizes the caller's slot, too: the call that warms a pass up is the call
 // that is captured next.
+//
+// `hold` keeps the pass's queues as they are until its launches are enqueued.
+struct PassHold {
+    std::unique_lock<std::mutex> slot, wide;
+};
+
 int pass_workspace(int dev, int slot, uint32_t npix, int spp, bool nrc, cudaStream_t stream, Tuning& tu,
-                   Workspace& ws) {
+                   Workspace& ws, PassHold& hold) {
+    if (slot < 0 || slot >= kWorkspaceSlots) return fail(TFG_E_INVALID, "render: workspace slot out of range");
+    hold.slot = std::unique_lock<std::mutex>(g_pass_mutex[dev][slot]);
     if (tu.widened) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         const cudaError_t e = cudaStreamIsCapturing(stream, &cap);
@@ -1265,6 +1278,7 @@ int pass_workspace(int dev, int slot, uint32_t npix, int spp, bool nrc, cudaStre
         if (e != cudaSuccess) cudaGetLastError();
         if (wide)
             if (int rc = ensure_workspace(dev, slot, npix, nrc, ws)) return rc;
+        if (wide) hold.wide = std::unique_lock<std::mutex>(g_pass_mutex[dev][kWideSlot]);
         size_t have = 0;
         {
             std::lock_guard<std::mutex> lk(g_ws_mutex);
@@ -1439,7 +1453,8 @@ int render_pass_ex(const TfgRenderParams& prm, const TfgCamara* d_cam, const Tfg
     if (int rc = require_sm100(dev)) return rc;
     Tuning tu = resolve_tuning(dev, (uint32_t)W * (uint32_t)H, prm.spp, nrc, nullptr);
     Workspace ws;
-    if (int rc = pass_workspace(dev, ws_slot, (uint32_t)W * (uint32_t)H, prm.spp, nrc, stream, tu, ws)) return rc;
+    PassHold hold;
+    if (int rc = pass_workspace(dev, ws_slot, (uint32_t)W * (uint32_t)H, prm.spp, nrc, stream, tu, ws, hold)) return rc;
     LaunchShapes sh;
     shapes_for(dev, sh);
     if (prepare_only) return ok();
@@ -1515,7 +1530,8 @@ int render_pass_multi(const TfgRenderParams& prm, const PassScene* scenes, int n
     const bool nrc = any_inf || train;
     Tuning tu = resolve_tuning(dev, (uint32_t)total, prm.spp, nrc, nullptr);
     Workspace ws;
-    if (int rc = pass_workspace(dev, ws_slot, (uint32_t)total, prm.spp, nrc, stream, tu, ws)) return rc;
+    PassHold hold;
+    if (int rc = pass_workspace(dev, ws_slot, (uint32_t)total, prm.spp, nrc, stream, tu, ws, hold)) return rc;
     LaunchShapes sh;
     shapes_for(dev, sh);
     if (prepare_only) return ok();
