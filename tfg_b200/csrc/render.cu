@@ -1090,6 +1090,22 @@ std::mutex g_ws_mutex;
 // takes two slots locks the wide one last.
 std::mutex g_pass_mutex[kMaxDevices][kWorkspaceSlots + 1];
 Workspace g_ws[kMaxDevices][kWorkspaceSlots + 1];
+// Largest wide wavefront asked for while the device's free memory bounded it (or
+// its allocation failed): smaller requests take what there is and neither query
+// the free memory nor try again.  Starts anew with every tuning set.
+size_t g_wide_asked[kMaxDevices] = {0};
+
+// Gives a slot's arrays back (cudaFree waits for work that uses them).
+void release_arrays(Workspace& w) {
+    void** arrays[] = {(void**)&w.ray[0], (void**)&w.ray[1], (void**)&w.hit, (void**)&w.shadow, (void**)&w.thr,
+                       (void**)&w.st, (void**)&w.lpre, (void**)&w.lsuf, (void**)&w.nrc, (void**)&w.ts};
+    for (void** a : arrays) {
+        if (*a) cudaFree(*a);
+        *a = nullptr;
+    }
+    w.cap = w.train_cap = 0;
+    ++w.generation;
+}
 
 int ensure_workspace(int dev, int slot, size_t paths, bool nrc, Workspace& out) {
     if (slot < 0 || slot > kWideSlot) return fail(TFG_E_INVALID, "render: workspace slot out of range");
@@ -1279,22 +1295,37 @@ int pass_workspace(int dev, int slot, uint32_t npix, int spp, bool nrc, cudaStre
         if (wide)
             if (int rc = ensure_workspace(dev, slot, npix, nrc, ws)) return rc;
         if (wide) hold.wide = std::unique_lock<std::mutex>(g_pass_mutex[dev][kWideSlot]);
-        size_t have = 0;
+        size_t have = 0, asked = 0;
         {
             std::lock_guard<std::mutex> lk(g_ws_mutex);
             have = g_ws[dev][kWideSlot].cap;
+            asked = g_wide_asked[dev];
         }
         if (wide && have < tu.wavefront) {
-            size_t free_b = 0, total_b = 0;
-            constexpr size_t kPathBytes = 2 * 32 + 16 + 64 + 5 * 16;
-            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); free_b = 0; }
-            const uint64_t fit = std::max<uint64_t>(free_b / 8 / kPathBytes, have);
+            uint64_t fit = have;
+            if (asked < tu.wavefront) {
+                size_t free_b = 0, total_b = 0;
+                constexpr size_t kPathBytes = 2 * 32 + 16 + 64 + 5 * 16;
+                if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); free_b = 0; }
+                fit = std::max<uint64_t>(free_b / 8 / kPathBytes, have);
+                asked = tu.wavefront;
+            }
             tu.wavefront = (uint32_t)std::min<uint64_t>(tu.wavefront, auto_wavefront(npix, spp, fit));
             wide = tu.wavefront > npix;
         }
         if (wide) {
-            if (ensure_workspace(dev, kWideSlot, tu.wavefront, nrc, ws) == 0) return ok();
+            const int rc = ensure_workspace(dev, kWideSlot, tu.wavefront, nrc, ws);
+            std::lock_guard<std::mutex> lk(g_ws_mutex);
+            if (rc == 0) {
+                if (tu.wavefront < asked) g_wide_asked[dev] = asked;
+                return ok();
+            }
             cudaGetLastError();
+            release_arrays(g_ws[dev][kWideSlot]);   // what it did get, before the fall-back
+        }
+        if (hold.wide) {
+            std::lock_guard<std::mutex> lk(g_ws_mutex);
+            g_wide_asked[dev] = std::max(g_wide_asked[dev], asked);
         }
         tu.wavefront = npix;
     }
@@ -1339,6 +1370,8 @@ int render_tuning_set(int dev, const TfgRenderTuning& t) {
     g_tune[dev] = t;
     g_tune_valid[dev] = true;
     ++g_tune_generation;
+    std::lock_guard<std::mutex> ws(g_ws_mutex);
+    g_wide_asked[dev] = 0;
     return ok();
 }
 
