@@ -333,7 +333,8 @@ typedef struct TfgRenderTuning {
                                    spread evenly over wavefronts of at most 2^24 paths and an eighth of
                                    the free device memory, at least one sample of every pixel (W*H) --
                                    exactly one under stream capture, for which an uncaptured call with
-                                   the same image size has made room.  More runs several samples of the
+                                   the same image size has made room.  Their queues stay allocated
+                                   until a tuning with wavefront_paths > 0 is set.  More runs several samples of the
                                    call per launch, less splits a sample into chunks; passes that query
                                    or train the cache stop at W*H.  0 or 1024 .. 2^26 (224 B of device
                                    memory per path) */

@@ -1,5 +1,5 @@
 """Device memory of widened wavefronts: at most an eighth of what is free, asked
-for once.  Run in processes of their own, whose queues start empty."""
+for once, and given back when a tuning names a wavefront size.  Run in processes of their own, whose queues start empty."""
 import subprocess
 import sys
 from pathlib import Path
@@ -59,6 +59,22 @@ print("fine")
 """
 
 
+_GIVEN_BACK = _COMMON + r"""
+before = free()
+assert taken(0) >= wide
+pt.set_tuning(pt.RenderTuning.default())
+assert before - free() >= wide                 # still the library's choice of size
+pt.set_tuning(pt.RenderTuning(wavefront_paths=W * H))
+assert before - free() <= 16 * MB, before - free()
+taken(1)
+pt.set_tuning(pt.RenderTuning.default())
+assert taken(2) >= wide
+for k in (1, 2):
+    assert torch.equal(accs[0], accs[k])
+print("fine")
+"""
+
+
 def _run(code):
     res = subprocess.run([sys.executable, "-c", code, str(ROOT)], capture_output=True, text=True, timeout=300)
     assert res.returncode == 0 and "fine" in res.stdout, res.stdout[-1000:] + res.stderr[-2000:]
@@ -66,3 +82,7 @@ def _run(code):
 
 def test_bounded_by_free_memory_and_asked_once(built):
     _run(_BOUNDED)
+
+
+def test_given_back_with_a_named_size(built):
+    _run(_GIVEN_BACK)

@@ -1332,6 +1332,20 @@ int pass_workspace(int dev, int slot, uint32_t npix, int spp, bool nrc, cudaStre
     return ensure_workspace(dev, slot, tu.wavefront, nrc, ws);
 }
 
+// Gives the widened queues back, once no pass on another thread is enqueueing on
+// them.  Another thread's stream capture is not disturbed: no captured pass uses
+// them.
+void release_wide_queues(int dev) {
+    std::lock_guard<std::mutex> pass(g_pass_mutex[dev][kWideSlot]);
+    std::lock_guard<std::mutex> lk(g_ws_mutex);
+    Workspace& w = g_ws[dev][kWideSlot];
+    if (w.cap == 0) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    release_arrays(w);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
 // Wavefronts up to kFewPaths paths run on k_few alone; longer ones have it
 // beside the long-queue kernels from bounce kFewFrom on.
 constexpr uint32_t kFewPaths = 65536;
@@ -1868,7 +1882,9 @@ extern "C" int tfgRenderTuningSet(const TfgRenderTuning* t) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return tfg::fail((int)e, cudaGetErrorString(e));
     if (int rc = tfg::require_sm100(dev)) return rc;
-    return tfg::render_tuning_set(dev, *t);
+    if (int rc = tfg::render_tuning_set(dev, *t)) return rc;
+    if (t->wavefront_paths > 0) tfg::release_wide_queues(dev);
+    return tfg::ok();
 }
 
 extern "C" int tfgRenderTuningGet(TfgRenderTuning* out) {
