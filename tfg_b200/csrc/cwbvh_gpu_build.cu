@@ -614,8 +614,11 @@ __global__ void k_emit_tris(const float* __restrict__ verts, const uint32_t* __r
 }
 
 // Pool of each device that builds' scratch blocks come from: stream-ordered,
-// keeping at most kPoolKeep bytes between builds (more goes back to the
-// device when a build's stream has been synchronised).  One block per build,
+// keeping at most kPoolKeep bytes between builds.  A pool gives what it holds
+// above that back at the next synchronisation after the memory was freed, so a
+// build frees its scratch before it synchronises for the last time (freed after
+// it, the 0.5 GB of a 2 M triangle build stayed until the program synchronised
+// again).  One block per build,
 // so builds on several threads or streams never share memory.
 constexpr uint64_t kPoolKeep = 128ull << 20;
 std::mutex g_pool_mutex;
@@ -645,7 +648,7 @@ cudaError_t build_pool(int dev, cudaMemPool_t* out) {
 }
 
 // One scratch block, carved into 256-byte aligned arrays; freed in stream
-// order on every exit path.
+// order, on an early exit with a synchronisation of its own.
 struct Scratch {
     cudaStream_t s;
     uint8_t* base = nullptr;
@@ -661,8 +664,15 @@ struct Scratch {
         used += pad(count * sizeof(T));
         return q;
     }
+    cudaError_t release() {
+        uint8_t* b = base;
+        base = nullptr;
+        return b ? cudaFreeAsync(b, s) : cudaSuccess;
+    }
     ~Scratch() {
-        if (base) cudaFreeAsync(base, s);
+        if (!base) return;
+        release();
+        cudaStreamSynchronize(s);
     }
 };
 
@@ -797,6 +807,8 @@ extern "C" int tfgTinyBVHConstruirGPU(const TfgPrimitiva* d_prims, int32_t n, Tf
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(out->ref.d_nodos, nodes, (size_t)num_nodes * 80, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = scan.release();
+    if (e == cudaSuccess) e = sc.release();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return bail(e);
     out->ref.num_nodos = num_nodes;
