@@ -428,7 +428,7 @@ __global__ void k_generate(PassArgs a, TableOf<MS> tab) {
 }
 
 // ------------------------------------------------------------------ trace
-template <int TRI_FMT, bool STATS, bool MS>
+template <int TRI_FMT, bool STATS, bool MS, bool TURNS = !MS>
 __global__ void __launch_bounds__(256, MS && !STATS ? 4 : 0) k_trace(PassArgs a, int bounce, TableOf<MS> tab) {
     extern __shared__ unsigned char smem_raw[];
     if (a.few_max) hand_over(a.ws.counters, bounce, 0);   // k_few, beside
@@ -458,10 +458,11 @@ __global__ void __launch_bounds__(256, MS && !STATS ? 4 : 0) k_trace(PassArgs a,
     // wait for the longest list.  1080p, 4 samples, 1.0 M triangles: 11.16 ->
     // 10.69 ms, 512 x 512 box 2.28 -> 2.27 ms (one triangle per turn 10.61 /
     // 2.30 ms, three 11.08 / 2.28).  The shadow stage and single coherent ray
-    // batches measured slower this way and keep step(), and so does the batch
-    // kernel, whose 64 registers do not hold the second loop.
+    // batches measured slower this way and keep step(), and so do small meshes
+    // (kStepTris) and the batch kernel, whose 64 registers do not hold the second
+    // loop.
     CwbvhRay<TRI_FMT, false> r;
-    r.tg.y = 0u;
+    if constexpr (TURNS) r.tg.y = 0u;
     uint32_t csc = 0;   // a batch: the current ray's scene, whose tree is looked up again at every step
     uint32_t cur = kMissId, bid = kMissId;
     float best = 0.0f, bu = 0.0f, bv = 0.0f;
@@ -493,7 +494,7 @@ __global__ void __launch_bounds__(256, MS && !STATS ? 4 : 0) k_trace(PassArgs a,
             if (cur != kMissId) g = geo_of<MS>(a, tab, csc);
         }
         bool done;
-        if constexpr (MS) {
+        if constexpr (!TURNS) {
             done = cur != kMissId && !(g.has_bvh && r.step(g.nodes, g.tris, st));
         } else {
             const bool act = cur != kMissId;
@@ -1174,6 +1175,7 @@ struct LaunchShapes {
     int sms = 0;
     // resident CTAs per SM: [one scene / batch][triangle format][64, 128, 256 threads]
     int trace_occ[2][2][3] = {};
+    int step_occ[2][3] = {};         // k_trace without turns: [triangle format][threads]
     int shadow_occ[2][2][3] = {};
     int shade_blocks[2] = {0, 0};
     int few_occ[2][2] = {};          // k_few: [one scene / batch][triangle format]
@@ -1201,6 +1203,8 @@ int shapes_for(int dev, LaunchShapes& s) {
             const size_t sm = trace_smem(kSmemPrims, bt), sm_ms = trace_smem(0, bt);
             g.trace_occ[0][0][k] = occ_of(k_trace<0, false, false>, bt, sm);
             g.trace_occ[0][1][k] = occ_of(k_trace<1, false, false>, bt, sm);
+            g.step_occ[0][k] = occ_of(k_trace<0, false, false, false>, bt, sm);
+            g.step_occ[1][k] = occ_of(k_trace<1, false, false, false>, bt, sm);
             g.shadow_occ[0][0][k] = occ_of(k_shadow<0, false, false>, bt, sm);
             g.shadow_occ[0][1][k] = occ_of(k_shadow<1, false, false>, bt, sm);
             g.trace_occ[1][0][k] = occ_of(k_trace<0, false, true>, bt, sm_ms);
@@ -1350,6 +1354,15 @@ void release_wide_queues(int dev) {
 // beside the long-queue kernels from bounce kFewFrom on.
 constexpr uint32_t kFewPaths = 65536;
 constexpr int kFewFrom = 2;
+
+// Wavefronts of at most kStepPaths paths over at most kStepTris triangles trace
+// with step() instead of turns: a ray meets few triangles there, and the turns'
+// reconvergence costs more than it gains.  One sample, turns / step: 400 x 300
+// in a box of 1,280 triangles 415 / 406 us, of 5,120 488 / 482, of 20,480
+// 599 / 598; 640 x 400 over terrain of 6,272 triangles 465 / 468, of 12,320
+// 492 / 502.  Four samples of 1024 x 576 in the box of 5,120: 3.866 / 3.875 ms.
+constexpr int kStepTris = 6000;
+constexpr uint32_t kStepPaths = 1u << 20;
 
 // Persistent traversal grid: every SM holds as many CTAs as fit, or the
 // tuned number of warps.
@@ -1604,7 +1617,9 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     const int ti = threads_index(tu.threads);
     const int bt = kThreadChoices[ti];
     const size_t smem = trace_smem(MS ? 0 : a.nprims, bt);
+    const bool small_mesh = !MS && a.nmesh <= kStepTris;
     const int trace_grid = persistent_grid(sh, sh.trace_occ[MS][fmt][ti], tu);
+    const int step_grid = persistent_grid(sh, sh.step_occ[fmt][ti], tu);
     const int shadow_grid = persistent_grid(sh, sh.shadow_occ[MS][fmt][ti], tu);
     const int shade_grid = sh.shade_blocks[MS];
     const Workspace& ws = a.ws;
@@ -1689,14 +1704,17 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
             if (e != cudaSuccess) return fail((int)e, std::string("render launch: ") + cudaGetErrorString(e));
             continue;
         }
+        const bool steps = small_mesh && a.nq <= kStepPaths;
         for (int b = 0; b < prm.max_depth; ++b) {
             a.few_max = few_ok && b >= kFewFrom ? few_groups : 0u;
             stage(1, [&] {
                 if (fmt == 0) {
                     if (counts) k_trace<0, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
+                    else if (steps) k_trace<0, false, MS, false><<<step_grid, bt, smem, stream>>>(a, b, tab);
                     else k_trace<0, false, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
                 } else {
                     if (counts) k_trace<1, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
+                    else if (steps) k_trace<1, false, MS, false><<<step_grid, bt, smem, stream>>>(a, b, tab);
                     else k_trace<1, false, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
                 }
                 if (a.few_max) few(b, -1, 0, few_groups, stream);
