@@ -169,7 +169,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // starts beside them: what earlier kernels wrote is promised to be visible to a
 // kernel that has waited (pdl_wait), and k_few cannot wait for a kernel that it
 // runs beside.  So the first block of the one writes length + 1 into a word of
-// its own (zeroed with the counters) with release semantics before it lets k_few
+// its own (zeroed by k_generate) with release semantics before it lets k_few
 // start, and every block of the other acquires it, which orders all its later
 // reads after all that the first kernel could see.  A block that finds the word
 // still zero waits for the kernel's end instead.  (4 samples of
@@ -424,7 +424,9 @@ __global__ void k_generate(PassArgs a, TableOf<MS> tab) {
             a.ws.nrc[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.ws.counters[0] = a.nq;
+    // the wavefront's queue lengths and words; all of its kernels come later
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < kCounterWords; i += blockDim.x) a.ws.counters[i] = i == 0 ? a.nq : 0u;
 }
 
 // ------------------------------------------------------------------ trace
@@ -1351,9 +1353,14 @@ void release_wide_queues(int dev) {
 }
 
 // Wavefronts up to kFewPaths paths run on k_few alone; longer ones have it
-// beside the long-queue kernels from bounce kFewFrom on.
+// beside the long-queue kernels from bounce kFewFrom on, or kFewFromCache where
+// the cache may end paths at their second vertex.  An empty pair of launches
+// costs ~2.5 us, which a closed scene (queues that stay long until Russian
+// roulette) pays for nothing: from bounce 2 / 3 / 4, 400 x 300 paths in a box of
+// 1,280 triangles, 5 bounces, 406 / 404 / 401 us; the same over 8,320 triangles
+// of terrain 362 / 363 / 391; a 720p cache frame 1.28 / 1.33 / 1.39 ms.
 constexpr uint32_t kFewPaths = 65536;
-constexpr int kFewFrom = 2;
+constexpr int kFewFrom = 3, kFewFromCache = 2;
 
 // Wavefronts of at most kStepPaths paths over at most kStepTris triangles trace
 // with step() instead of turns: a ray meets few triangles there, and the turns'
@@ -1645,7 +1652,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     cudaStream_t sstream = overlap ? ws.side : stream;
     // k_few for short queues: alone, closest hits and the previous bounce's
     // shadow rays in one launch, for wavefronts that start short; beside the
-    // long-queue kernels from bounce kFewFrom on otherwise (the queue lengths
+    // long-queue kernels from the third or fourth bounce on otherwise (the queue lengths
     // are only known on the device).  There it starts beside the kernel whose
     // short queues it takes and waits for that one's end only at its own:
     // launched after it, the empty launches of a 20-bounce 906 x 562 sample cost
@@ -1688,8 +1695,6 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
         const int gen_blocks = (int)std::max<uint32_t>(1u, std::min<uint32_t>((a.nq + 255) / 256, (uint32_t)sh.sms * 8u));
         const uint32_t resolve_n = std::min(a.nq, N);
         const int res_blocks = (int)std::max<uint32_t>(1u, std::min<uint32_t>((resolve_n + 255) / 256, (uint32_t)sh.sms * 8u));
-        e = cudaMemsetAsync(ws.counters, 0, kCounterWords * sizeof(uint32_t), stream);
-        if (e != cudaSuccess) return fail((int)e, cudaGetErrorString(e));
         a.few_max = 0;
         stage(0, [&] { k_generate<MS><<<gen_blocks, 256, 0, stream>>>(a, tab); });
         if (few_ok && a.nq <= kFewPaths) {
@@ -1706,7 +1711,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
         }
         const bool steps = small_mesh && a.nq <= kStepPaths;
         for (int b = 0; b < prm.max_depth; ++b) {
-            a.few_max = few_ok && b >= kFewFrom ? few_groups : 0u;
+            a.few_max = few_ok && b >= (a.use_inf ? kFewFromCache : kFewFrom) ? few_groups : 0u;
             stage(1, [&] {
                 if (fmt == 0) {
                     if (counts) k_trace<0, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
