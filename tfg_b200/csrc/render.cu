@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(256, MS && !STATS ? 4 : 0) k_trace(PassArgs a,
     // 10.69 ms, 512 x 512 box 2.28 -> 2.27 ms (one triangle per turn 10.61 /
     // 2.30 ms, three 11.08 / 2.28).  The shadow stage and single coherent ray
     // batches measured slower this way and keep step(), and so do small meshes
-    // (kStepTris) and the batch kernel, whose 64 registers do not hold the second
+    // (kSmallTris) and the batch kernel, whose 64 registers do not hold the second
     // loop.
     CwbvhRay<TRI_FMT, false> r;
     if constexpr (TURNS) r.tg.y = 0u;
@@ -1352,23 +1352,32 @@ void release_wide_queues(int dev) {
     cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
-// Wavefronts up to kFewPaths paths run on k_few alone; longer ones have it
-// beside the long-queue kernels from bounce kFewFrom on, or kFewFromCache where
-// the cache may end paths at their second vertex.  An empty pair of launches
-// costs ~2.5 us, which a closed scene (queues that stay long until Russian
-// roulette) pays for nothing: from bounce 2 / 3 / 4, 400 x 300 paths in a box of
-// 1,280 triangles, 5 bounces, 406 / 404 / 401 us; the same over 8,320 triangles
-// of terrain 362 / 363 / 391; a 720p cache frame 1.28 / 1.33 / 1.39 ms.
-constexpr uint32_t kFewPaths = 65536;
+// Meshes of at most kSmallTris triangles: a ray meets few nodes and triangles.
+constexpr int kSmallTris = 6000;
+
+// Wavefronts up to kFewPaths paths run on k_few alone, over larger meshes (long
+// traversals, from which eight lanes gain more) up to kFewPathsMesh.  One sample
+// of 5 bounces, beside the long-queue kernels / alone: box of 1,280 triangles
+// 38,400 paths 279 / 224 us, 60,000 291 / 296, 76,800 316 / 350; box of 81,920
+// triangles 76,800 paths 590 / 490, 86,400 655 / 537, 120,000 744 / 683; terrain
+// of 12,320 triangles 86,400 paths 348 / 355 (10 bounces 475 / 456), 120,000
+// 367 / 441.
+constexpr uint32_t kFewPaths = 65536, kFewPathsMesh = 98304;
+
+// Longer ones have it beside the long-queue kernels from bounce kFewFrom on, or
+// kFewFromCache where the cache may end paths at their second vertex.  An empty
+// pair of launches costs ~2.5 us, which a closed scene (queues that stay long
+// until Russian roulette) pays for nothing: from bounce 2 / 3 / 4, 400 x 300
+// paths in a box of 1,280 triangles, 5 bounces, 406 / 404 / 401 us; the same over
+// 8,320 triangles of terrain 362 / 363 / 391; a 720p cache frame
+// 1.28 / 1.33 / 1.39 ms.
 constexpr int kFewFrom = 3, kFewFromCache = 2;
 
-// Wavefronts of at most kStepPaths paths over at most kStepTris triangles trace
-// with step() instead of turns: a ray meets few triangles there, and the turns'
-// reconvergence costs more than it gains.  One sample, turns / step: 400 x 300
+// Wavefronts of at most kStepPaths paths over a small mesh trace with step()
+// instead of turns, whose reconvergence costs more there than it gains.  One sample, turns / step: 400 x 300
 // in a box of 1,280 triangles 415 / 406 us, of 5,120 488 / 482, of 20,480
 // 599 / 598; 640 x 400 over terrain of 6,272 triangles 465 / 468, of 12,320
 // 492 / 502.  Four samples of 1024 x 576 in the box of 5,120: 3.866 / 3.875 ms.
-constexpr int kStepTris = 6000;
 constexpr uint32_t kStepPaths = 1u << 20;
 
 // Persistent traversal grid: every SM holds as many CTAs as fit, or the
@@ -1624,7 +1633,8 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     const int ti = threads_index(tu.threads);
     const int bt = kThreadChoices[ti];
     const size_t smem = trace_smem(MS ? 0 : a.nprims, bt);
-    const bool small_mesh = !MS && a.nmesh <= kStepTris;
+    const bool small_mesh = !MS && a.nmesh <= kSmallTris;
+    const uint32_t few_paths = MS || small_mesh ? kFewPaths : kFewPathsMesh;
     const int trace_grid = persistent_grid(sh, sh.trace_occ[MS][fmt][ti], tu);
     const int step_grid = persistent_grid(sh, sh.step_occ[fmt][ti], tu);
     const int shadow_grid = persistent_grid(sh, sh.shadow_occ[MS][fmt][ti], tu);
@@ -1697,7 +1707,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
         const int res_blocks = (int)std::max<uint32_t>(1u, std::min<uint32_t>((resolve_n + 255) / 256, (uint32_t)sh.sms * 8u));
         a.few_max = 0;
         stage(0, [&] { k_generate<MS><<<gen_blocks, 256, 0, stream>>>(a, tab); });
-        if (few_ok && a.nq <= kFewPaths) {
+        if (few_ok && a.nq <= few_paths) {
             for (int b = 0; b < prm.max_depth; ++b) {
                 few(b, b - 1, 1, (b == 0 ? 1u : 1u + few_points) * a.nq, stream);
                 launch(k_shade<MS>, std::min((uint32_t)shade_grid, (a.nq + kShadeThreads - 1u) / kShadeThreads),
