@@ -48,9 +48,9 @@ def test_no_other_training_kernel_is_launched_early():
     assert names == {"k_train", "k_train128", "k_wgrad", "k_adam", "k_adam_hash"}
 
 
-@pytest.mark.parametrize("kernel", ["k_shade", "k_resolve"])
-def test_render_kernels_wait_first(kernel):
-    assert _touched_before_wait(_body((CSRC / "render.cu").read_text(), kernel), "pdl_sync") == []
+@pytest.mark.parametrize("kernel,wait", [("k_shade", "pdl_sync"), ("k_resolve", "pdl_sync"), ("k_trace", "pdl_wait")])
+def test_render_kernels_wait_first(kernel, wait):
+    assert _touched_before_wait(_body((CSRC / "render.cu").read_text(), kernel), wait) == []
 
 
 def test_short_queue_kernel_waits_or_acquires_first():
@@ -73,4 +73,4 @@ def test_short_queue_kernel_waits_or_acquires_first():
 
 def test_no_other_render_kernel_is_launched_early():
     src = (CSRC / "render.cu").read_text()
-    assert set(re.findall(r"[ (]launch\((\w+)<", src)) == {"k_few", "k_shade", "k_resolve"}
+    assert set(re.findall(r"[ (]launch\((\w+)<", src)) == {"k_few", "k_shade", "k_resolve", "k_trace"}

@@ -150,8 +150,9 @@ struct Outs {
 };
 
 // ------------------------------------------------------------------ helpers
-// Kernels of a short wavefront are launched with programmatic stream
-// serialisation: each starts while the one before it ends and waits for it here
+// Kernels are launched with programmatic stream serialisation (a short
+// wavefront's all, a long one's k_trace, k_shade and k_few):
+// each starts while the one before it ends and waits for it here
 // before it touches global memory; then it lets its own successor start, so that
 // by the time any kernel runs, all but its predecessor have finished.  Both
 // calls do nothing in kernels launched the ordinary way.  A 128 x 128 sample of
@@ -165,7 +166,7 @@ __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.laun
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Handover of a queue's length from k_trace / k_shadow, which start in stream
-// order and so see all that was written before them, to the k_few launch that
+// order or have waited and so see all that was written before them, to the k_few launch that
 // starts beside them: what earlier kernels wrote is promised to be visible to a
 // kernel that has waited (pdl_wait), and k_few cannot wait for a kernel that it
 // runs beside.  So the first block of the one writes length + 1 into a word of
@@ -433,6 +434,7 @@ __global__ void k_generate(PassArgs a, TableOf<MS> tab) {
 template <int TRI_FMT, bool STATS, bool MS, bool TURNS = !MS>
 __global__ void __launch_bounds__(256, MS && !STATS ? 4 : 0) k_trace(PassArgs a, int bounce, TableOf<MS> tab) {
     extern __shared__ unsigned char smem_raw[];
+    pdl_wait();
     if (a.few_max) hand_over(a.ws.counters, bounce, 0);   // k_few, beside
     uint2* sstack = reinterpret_cast<uint2*>(smem_raw);
     APrim* sprims = reinterpret_cast<APrim*>(smem_raw + sizeof(uint2) * kSmemStack * blockDim.x);
@@ -1667,18 +1669,23 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     // short queues it takes and waits for that one's end only at its own:
     // launched after it, the empty launches of a 20-bounce 906 x 562 sample cost
     // 52 us of 1,356.
+    // Long wavefronts launch k_trace and k_shade early, too: a boundary between two
+    // kernels costs 1 to 2 us less (one sample of 400 x 300 paths in a box of 1,280
+    // triangles, 5 bounces, 400 -> 392 us, of 81,920 746 -> 738; 720p cache frame
+    // 1.275 -> 1.26 ms; 4 samples of 1080p 10.38 -> 10.36).
     // Stage timing and work counts keep the stages apart.
     const uint32_t few_groups = (uint32_t)(sh.sms * sh.few_occ[MS][fmt]) * (kFewThreads / 8u);
     const bool few_ok = !times && !counts;
     const uint32_t few_points = MS || a.nlights <= 1 ? 1u : a.nlights <= 2 ? 2u : 4u;   // groups per shading point
     // `early`: with programmatic stream serialisation (pdl_sync)
-    auto launch = [&](auto kernel, uint32_t grid, uint32_t threads, cudaStream_t st, bool early, auto... args) {
+    auto launch = [&](auto kernel, uint32_t grid, uint32_t threads, size_t dyn_smem, cudaStream_t st, bool early, auto... args) {
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr.val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(grid);
         cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = dyn_smem;
         cfg.stream = st;
         cfg.attrs = &attr;
         cfg.numAttrs = early ? 1 : 0;
@@ -1687,8 +1694,8 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     auto few = [&](int tb, int sb, int always, uint32_t tasks, cudaStream_t st) {
         const uint32_t fit = (uint32_t)(sh.sms * sh.few_occ[MS][fmt]);
         const uint32_t grid = std::max(1u, std::min(fit, (tasks + kFewThreads / 8u - 1) / (kFewThreads / 8u)));
-        if (fmt == 0) launch(k_few<0, MS>, grid, kFewThreads, st, true, a, tb, sb, always, tab);
-        else launch(k_few<1, MS>, grid, kFewThreads, st, true, a, tb, sb, always, tab);
+        if (fmt == 0) launch(k_few<0, MS>, grid, kFewThreads, 0, st, true, a, tb, sb, always, tab);
+        else launch(k_few<1, MS>, grid, kFewThreads, 0, st, true, a, tb, sb, always, tab);
     };
     a.frame = frame;
     a.img = img;
@@ -1711,10 +1718,10 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
             for (int b = 0; b < prm.max_depth; ++b) {
                 few(b, b - 1, 1, (b == 0 ? 1u : 1u + few_points) * a.nq, stream);
                 launch(k_shade<MS>, std::min((uint32_t)shade_grid, (a.nq + kShadeThreads - 1u) / kShadeThreads),
-                       (uint32_t)kShadeThreads, stream, true, a, b, tab);
+                       (uint32_t)kShadeThreads, 0, stream, true, a, b, tab);
             }
             few(-1, prm.max_depth - 1, 1, few_points * a.nq, stream);
-            launch(k_resolve<MS>, (uint32_t)res_blocks, 256u, stream, true, a, tab);
+            launch(k_resolve<MS>, (uint32_t)res_blocks, 256u, 0, stream, true, a, tab);
             e = cudaGetLastError();
             if (e != cudaSuccess) return fail((int)e, std::string("render launch: ") + cudaGetErrorString(e));
             continue;
@@ -1723,14 +1730,15 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
         for (int b = 0; b < prm.max_depth; ++b) {
             a.few_max = few_ok && b >= (a.use_inf ? kFewFromCache : kFewFrom) ? few_groups : 0u;
             stage(1, [&] {
-                if (fmt == 0) {
-                    if (counts) k_trace<0, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
-                    else if (steps) k_trace<0, false, MS, false><<<step_grid, bt, smem, stream>>>(a, b, tab);
-                    else k_trace<0, false, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
+                if (counts) {
+                    if (fmt == 0) k_trace<0, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
+                    else k_trace<1, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
+                } else if (steps) {
+                    if (fmt == 0) launch(k_trace<0, false, MS, false>, step_grid, bt, smem, stream, few_ok, a, b, tab);
+                    else launch(k_trace<1, false, MS, false>, step_grid, bt, smem, stream, few_ok, a, b, tab);
                 } else {
-                    if (counts) k_trace<1, true, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
-                    else if (steps) k_trace<1, false, MS, false><<<step_grid, bt, smem, stream>>>(a, b, tab);
-                    else k_trace<1, false, MS><<<trace_grid, bt, smem, stream>>>(a, b, tab);
+                    if (fmt == 0) launch(k_trace<0, false, MS>, trace_grid, bt, smem, stream, few_ok, a, b, tab);
+                    else launch(k_trace<1, false, MS>, trace_grid, bt, smem, stream, few_ok, a, b, tab);
                 }
                 if (a.few_max) few(b, -1, 0, few_groups, stream);
             });
@@ -1738,7 +1746,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
                 e = cudaStreamWaitEvent(stream, ws.join[b - 1], 0);
                 if (e != cudaSuccess) return fail((int)e, cudaGetErrorString(e));
             }
-            stage(2, [&] { k_shade<MS><<<shade_grid, kShadeThreads, 0, stream>>>(a, b, tab); });
+            stage(2, [&] { launch(k_shade<MS>, shade_grid, kShadeThreads, 0, stream, few_ok, a, b, tab); });
             if (overlap) {
                 e = cudaEventRecord(ws.fork[b], stream);
                 if (e == cudaSuccess) e = cudaStreamWaitEvent(sstream, ws.fork[b], 0);
