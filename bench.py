@@ -49,10 +49,11 @@ AUTO_PATHS = 1 << 24
 # (lts__t_bytes.sum) per closest-hit ray traced, the share of issue slots
 # used (sm__inst_issued.avg.per_cycle_active / 4) and the SIMT efficiency
 # (smsp__thread_inst_executed_per_inst_executed.ratio / 32), over the pass's
-# 4,001,265 rays, weighted by duration and by instructions respectively.
-TRACE_L2_BYTES_PER_RAY = 508.0
-TRACE_ISSUE_FRAC = 0.561
-TRACE_SIMT_EFFICIENCY = 0.406
+# 4,001,265 rays, weighted by duration and by instructions respectively (the last
+# three bounces' rays, at most 1.4 %, are the short-queue kernel's).
+TRACE_L2_BYTES_PER_RAY = 512.0
+TRACE_ISSUE_FRAC = 0.656
+TRACE_SIMT_EFFICIENCY = 0.480
 # k_shadow's active lanes per instruction (of 32) on the first bounce of the
 # one-sample pass (profiles/k_trace_k_shadow_bounce0_full_1080p.md: 15.18).
 SHADOW_SIMT_EFFICIENCY = 0.474

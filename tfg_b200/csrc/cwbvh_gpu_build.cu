@@ -25,7 +25,7 @@
 // A build is a chain of short dependent kernels, so what counts is the host
 // work around them and each kernel's latency: all scratch is one block of a
 // bounded stream-ordered pool (cudaMalloc and cudaFree take ~0.3 ms each here:
-// the former 25 pairs took most of the 5.8 ms of an 81,920-triangle build),
+// the former 25 pairs took most of an 81,920-triangle build),
 // the result is one allocation made while the GPU works, the initial values
 // come from a kernel, and the levels run in batches whose sizes stay on the
 // device (one host read per eight levels instead of one per level).
