@@ -51,3 +51,39 @@ def test_primitives_that_are_not_finite(built, w, h, bad):
     got, want = _both(s, pt.TRIS_WATERTIGHT, depth=8)
     assert want.any()
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.fixture
+def default_tuning():
+    yield
+    pt.set_tuning(pt.RenderTuning.default())
+
+
+# queues that stay long and queues that become short, on one stream and on two,
+# directly and replayed from a graph: the kernels start early either way
+@pytest.mark.parametrize("overlap", [0, 1])
+@pytest.mark.parametrize("build", [lambda w, h: scenes.box_icosphere(w, h, subdiv=4),
+                                   lambda w, h: scenes.spheres_terrain(w, h, subdiv=2, terrain_n=60)])
+def test_early_launches_on_one_stream_and_two(built, default_tuning, build, overlap):
+    w, h = 400, 301
+    s = build(w, h)
+    want = _both(s, pt.TRIS_WATERTIGHT, depth=9)[1]
+    ds = pt.DeviceScene(s, "cuda")
+    p = pt.RenderParams(max_depth=9, rr_min_depth=3, shadow_mesh=1, tri_format=pt.TRIS_WATERTIGHT, spp=1, accumulate=1)
+    pt.set_tuning(pt.RenderTuning(overlap_shadow=overlap))
+    accs = [torch.zeros(w * h * 3, device="cuda") for _ in range(4)]
+    for acc in accs:   # back to back
+        pt.render_pass(ds, p, 3, None, acc)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            accs[0].zero_()
+            pt.render_pass(ds, p, 3, None, accs[0])
+        for _ in range(3):
+            graph.replay()
+        stream.synchronize()
+    for acc in accs:
+        np.testing.assert_array_equal(acc.cpu().numpy(), want)
+    ds.close()
