@@ -1357,14 +1357,14 @@ void release_wide_queues(int dev) {
 // Meshes of at most kSmallTris triangles: a ray meets few nodes and triangles.
 constexpr int kSmallTris = 6000;
 
-// Wavefronts up to kFewPaths paths run on k_few alone, over larger meshes (long
-// traversals, from which eight lanes gain more) up to kFewPathsMesh.  One sample
-// of 5 bounces, beside the long-queue kernels / alone: box of 1,280 triangles
-// 38,400 paths 279 / 224 us, 60,000 291 / 296, 76,800 316 / 350; box of 81,920
-// triangles 76,800 paths 590 / 490, 86,400 655 / 537, 120,000 744 / 683; terrain
-// of 12,320 triangles 86,400 paths 348 / 355 (10 bounces 475 / 456), 120,000
-// 367 / 441.
-constexpr uint32_t kFewPaths = 65536, kFewPathsMesh = 98304;
+// Wavefronts up to kFewPaths paths run on k_few alone.  One sample of 5 bounces,
+// beside the long-queue kernels / alone: box of 1,280 triangles 38,400 paths
+// 279 / 224 us, 60,000 291 / 296, 76,800 316 / 350; terrain of 8,320 triangles
+// 76,800 paths 306 / 322, of 65,480 365 / 379.  (Closed scenes with long
+// traversals and deep ones would gain further up: box of 81,920 triangles 76,800
+// paths 596 / 489, terrain of 65,480 at 96,000 paths 8 bounces 473 / 502, 20
+// bounces 641 / 587.)
+constexpr uint32_t kFewPaths = 65536;
 
 // Longer ones have it beside the long-queue kernels from bounce kFewFrom on, or
 // kFewFromCache where the cache may end paths at their second vertex.  An empty
@@ -1636,7 +1636,6 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
     const int bt = kThreadChoices[ti];
     const size_t smem = trace_smem(MS ? 0 : a.nprims, bt);
     const bool small_mesh = !MS && a.nmesh <= kSmallTris;
-    const uint32_t few_paths = MS || small_mesh ? kFewPaths : kFewPathsMesh;
     const int trace_grid = persistent_grid(sh, sh.trace_occ[MS][fmt][ti], tu);
     const int step_grid = persistent_grid(sh, sh.step_occ[fmt][ti], tu);
     const int shadow_grid = persistent_grid(sh, sh.shadow_occ[MS][fmt][ti], tu);
@@ -1714,7 +1713,7 @@ int enqueue_pass(PassArgs a, const TableOf<MS>& tab, const TfgRenderParams& prm,
         const int res_blocks = (int)std::max<uint32_t>(1u, std::min<uint32_t>((resolve_n + 255) / 256, (uint32_t)sh.sms * 8u));
         a.few_max = 0;
         stage(0, [&] { k_generate<MS><<<gen_blocks, 256, 0, stream>>>(a, tab); });
-        if (few_ok && a.nq <= few_paths) {
+        if (few_ok && a.nq <= kFewPaths) {
             for (int b = 0; b < prm.max_depth; ++b) {
                 few(b, b - 1, 1, (b == 0 ? 1u : 1u + few_points) * a.nq, stream);
                 launch(k_shade<MS>, std::min((uint32_t)shade_grid, (a.nq + kShadeThreads - 1u) / kShadeThreads),
