@@ -151,10 +151,10 @@ struct Outs {
 
 // ------------------------------------------------------------------ helpers
 // Kernels are launched with programmatic stream serialisation (a short
-// wavefront's all, a long one's k_trace, k_shade and k_few):
-// each starts while the one before it ends and waits for it here
-// before it touches global memory; then it lets its own successor start, so that
-// by the time any kernel runs, all but its predecessor have finished.  Both
+// wavefront's all but the first, a long one's k_trace, k_shade and k_few): each
+// starts while the one before it ends and waits for it here before it touches
+// global memory; then it lets its own successor start, so that by the time any
+// kernel runs, all but its predecessor have finished.  Both
 // calls do nothing in kernels launched the ordinary way.  A 128 x 128 sample of
 // 20 bounces is 43 kernels of 4 to 19 us: 430 us with ordinary launches, 348 us
 // so.  k_generate does not let its successor in early: 7 us more.
@@ -166,8 +166,8 @@ __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.laun
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Handover of a queue's length from k_trace / k_shadow, which start in stream
-// order or have waited and so see all that was written before them, to the k_few launch that
-// starts beside them: what earlier kernels wrote is promised to be visible to a
+// order or have waited and so see all that was written before them, to the k_few
+// launch that starts beside them: what earlier kernels wrote is promised to be visible to a
 // kernel that has waited (pdl_wait), and k_few cannot wait for a kernel that it
 // runs beside.  So the first block of the one writes length + 1 into a word of
 // its own (zeroed by k_generate) with release semantics before it lets k_few
@@ -1376,10 +1376,11 @@ constexpr uint32_t kFewPaths = 65536;
 constexpr int kFewFrom = 3, kFewFromCache = 2;
 
 // Wavefronts of at most kStepPaths paths over a small mesh trace with step()
-// instead of turns, whose reconvergence costs more there than it gains.  One sample, turns / step: 400 x 300
-// in a box of 1,280 triangles 415 / 406 us, of 5,120 488 / 482, of 20,480
-// 599 / 598; 640 x 400 over terrain of 6,272 triangles 465 / 468, of 12,320
-// 492 / 502.  Four samples of 1024 x 576 in the box of 5,120: 3.866 / 3.875 ms.
+// instead of turns, whose reconvergence costs more there than it gains.  One
+// sample, turns / step: 400 x 300 in a box of 1,280 triangles 415 / 406 us, of
+// 5,120 488 / 482, of 20,480 599 / 598; 640 x 400 over terrain of 6,272
+// triangles 465 / 468, of 12,320 492 / 502.  Four samples of 1024 x 576 in the
+// box of 5,120: 3.866 / 3.875 ms.
 constexpr uint32_t kStepPaths = 1u << 20;
 
 // Persistent traversal grid: every SM holds as many CTAs as fit, or the
